@@ -453,7 +453,7 @@ struct cpic_adj {
 	Scale *sc;
 	double *part, *loss_d, *stage;
 	void *twx, *twy;
-	double *cosx, *cosy;
+	void *green;              // Green's function, column order (T)
 	int nckpt;
 	bool have_forward;
 	double loss;
@@ -496,7 +496,7 @@ void solve_E(cpic_adj *a, T *Ex, T *Ey)
 		mean = a->rsum;
 	}
 	poisson_launch<T>(a->fg, a->rho, a->qinv, mean, P<C>(a->spec), P<C>(a->twx), P<C>(a->twy),
-			a->cosx, a->cosy, P<T>(a->phi), a->st);
+			P<T>(a->phi), a->st, P<T>(a->green));
 	k_E<T><<<blocks_for(a->ng), 256, 0, a->st>>>(a->g, P<T>(a->phi), Ex, Ey);
 }
 
@@ -535,8 +535,8 @@ void grid_adjoint(cpic_adj *a)
 {
 	typedef typename Cx<T>::t C;
 	k_div<T><<<blocks_for(a->ng), 256, 0, a->st>>>(a->g, P<T>(a->Ebx), P<T>(a->Eby), P<T>(a->phi));
-	poisson_launch_real<T>(a->fg, P<T>(a->phi), P<C>(a->spec), P<C>(a->twx), P<C>(a->twy),
-			a->cosx, a->cosy, P<T>(a->rhob), a->st);
+	poisson_launch_real<T>(a->g.nx, a->g.ny, P<T>(a->phi), P<C>(a->spec), P<C>(a->twx), P<C>(a->twy),
+			P<T>(a->green), P<T>(a->rhob), a->st);
 	k_absmax<T><<<blocks_for(a->ng), 256, 0, a->st>>>(a->ng, P<T>(a->rhob), a->sc);
 }
 
@@ -662,6 +662,7 @@ CPIC_API int cpic_adj_create(const cpic_adj_params_t *p, int64_t n, cpic_adj_t *
 	int K = (int) a->p.checkpoint_every;
 	a->nckpt = (int) ((p->nsteps + K - 1) / K);
 	int64_t ng = a->ng, nh = p->nx / 2 + 1;
+	double *cosx = nullptr, *cosy = nullptr;
 	size_t ts = a->ts, cs = 2 * ts;
 	int r = CPIC_OK;
 	if(cudaStreamCreateWithFlags(&a->st, cudaStreamNonBlocking) != cudaSuccess)
@@ -687,7 +688,8 @@ CPIC_API int cpic_adj_create(const cpic_adj_params_t *p, int64_t n, cpic_adj_t *
 	AL(a->loss_d, sizeof(double));
 	AL(a->stage, 4 * n * sizeof(double));
 	AL(a->twx, p->nx / 2 * cs); AL(a->twy, p->ny / 2 * cs);
-	AL(a->cosx, p->nx * sizeof(double)); AL(a->cosy, p->ny * sizeof(double));
+	AL(a->green, (size_t) nh * p->ny * ts);
+	AL(cosx, p->nx * sizeof(double)); AL(cosy, p->ny * sizeof(double));
 #undef AL
 	{
 		// Green's function cosines (solver.c:257-278) and twiddles, as the
@@ -695,8 +697,12 @@ CPIC_API int cpic_adj_create(const cpic_adj_params_t *p, int64_t n, cpic_adj_t *
 		std::vector<double> cx(p->nx), cy(p->ny);
 		for(int64_t i = 0; i < p->nx; i++) cx[i] = cos(2.0 * M_PI / p->nx * i);
 		for(int64_t i = 0; i < p->ny; i++) cy[i] = cos(2.0 * M_PI / p->ny * i);
-		cudaMemcpy(a->cosx, cx.data(), p->nx * sizeof(double), cudaMemcpyHostToDevice);
-		cudaMemcpy(a->cosy, cy.data(), p->ny * sizeof(double), cudaMemcpyHostToDevice);
+		cudaMemcpy(cosx, cx.data(), p->nx * sizeof(double), cudaMemcpyHostToDevice);
+		cudaMemcpy(cosy, cy.data(), p->ny * sizeof(double), cudaMemcpyHostToDevice);
+		if(a->f64) k_green<double><<<blocks_for(nh * p->ny), 256>>>(a->g.nx, a->g.ny, cosx, cosy,
+				P<double>(a->green));
+		else k_green<float><<<blocks_for(nh * p->ny), 256>>>(a->g.nx, a->g.ny, cosx, cosy,
+				P<float>(a->green));
 		for(int dim = 0; dim < 2; dim++)
 		{
 			int64_t m = dim == 0 ? p->nx : p->ny;
@@ -720,7 +726,7 @@ CPIC_API int cpic_adj_create(const cpic_adj_params_t *p, int64_t n, cpic_adj_t *
 					(const void *) k_rows_inv<double>, (const void *) k_rows_fwd_real<double>,
 					(const void *) k_rows_fwd<float>, (const void *) k_cols<float>,
 					(const void *) k_rows_inv<float>, (const void *) k_rows_fwd_real<float>},
-					200 * 1024);
+					kFftMaxSmem);
 		});
 		if(e != cudaSuccess)
 		{
@@ -730,9 +736,13 @@ CPIC_API int cpic_adj_create(const cpic_adj_params_t *p, int64_t n, cpic_adj_t *
 		}
 	}
 	if(cudaDeviceSynchronize() != cudaSuccess) { r = CPIC_ECUDA; goto fail; }
+	cudaFree(cosx);
+	cudaFree(cosy);
 	*out = a;
 	return CPIC_OK;
 fail:
+	cudaFree(cosx);
+	cudaFree(cosy);
 	cpic_adj_destroy(a);
 	return r;
 }
@@ -742,7 +752,7 @@ CPIC_API void cpic_adj_destroy(cpic_adj_t *a)
 	if(!a) return;
 	void *bufs[] = {a->x, a->y, a->ux, a->uy, a->pbx, a->pby, a->ubx, a->uby, a->ckpt, a->hist,
 		a->histE, a->Ex, a->Ey, a->phi, a->rhob, a->Ebx, a->Eby, a->spec, a->rho, a->Ebfix,
-		a->rsum, a->sc, a->part, a->loss_d, a->stage, a->twx, a->twy, a->cosx, a->cosy};
+		a->rsum, a->sc, a->part, a->loss_d, a->stage, a->twx, a->twy, a->green};
 	for(void *b : bufs) if(b) cudaFree(b);
 	for(int i = 0; i < 4; i++) if(a->ev[i]) cudaEventDestroy(a->ev[i]);
 	if(a->st) cudaStreamDestroy(a->st);

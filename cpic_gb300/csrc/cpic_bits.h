@@ -14,6 +14,7 @@
 // on edge cases and random values.
 #pragma once
 #include <climits>
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 
@@ -101,6 +102,24 @@ CPIC_HD bool abs_gt(double d, double u)
 CPIC_HD bool is_finite(double d)
 {
 	return (to_bits(d) & 0x7ff0000000000000ull) != 0x7ff0000000000000ull;
+}
+
+// a / d for a finite d and its rounded reciprocal r = rn(1 / d), by
+// Markstein's method (IBM J. Res. Dev. 34, 1990): the quotient estimate a r
+// corrected once by its exact remainder, which gives the correctly rounded
+// quotient for every normal result.  Three fused or plain FP64
+// instructions for a division by a constant.  An infinite or NaN estimate is
+// returned as it is, as a / d would be.
+CPIC_HD double div_by(double a, double d, double r)
+{
+#ifdef __CUDA_ARCH__
+	const double q = __dmul_rn(a, r);
+	const double c = __fma_rn(__fma_rn(-q, d, a), r, q);
+#else
+	const double q = a * r;
+	const double c = std::fma(std::fma(-q, d, a), r, q);
+#endif
+	return is_finite(q) ? c : q;
 }
 
 // Division of a tile index by the number of tiles per row without a divide

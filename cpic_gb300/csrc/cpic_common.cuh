@@ -490,9 +490,8 @@ int push_f64_blocks_per_sm(size_t smem, int ppt);
 void launch_spill_f64(const SpillArgs &a, cudaStream_t s);
 void launch_E_f64(const Grid &g, const double *phi, double *Ex, double *Ey, cudaStream_t s);
 cudaError_t launch_poisson_f64(const Grid &g, const long long *rho, double qinv,
-		double2 *spec, const double2 *twx, const double2 *twy, const double *cosx,
-		const double *cosy, double *phi, cudaStream_t s, const long long *rho_lo, double qinv_lo,
-		const double *Gt);
+		double2 *spec, const double2 *twx, const double2 *twy, double *phi, cudaStream_t s,
+		const long long *rho_lo, double qinv_lo, const double *Gt);
 
 cudaError_t launch_push_mix(const PushArgs &a, int ntiles, size_t smem, int ppt, cudaStream_t s);
 // resident blocks per SM of the mixed fused kernel at this dynamic shared
@@ -501,6 +500,6 @@ int push_mix_blocks_per_sm(size_t smem, bool ids, int ppt, bool gp2);
 void launch_spill_mix(const SpillArgs &a, cudaStream_t s);
 void launch_E_mix(const Grid &g, const float *phi, float2 *E, cudaStream_t s);
 cudaError_t launch_poisson_mix(const Grid &g, const long long *rho, double qinv, const long long *rsum,
-		float2 *spec, const float2 *twx, const float2 *twy, const double *cosx,
-		const double *cosy, float *phi, cudaStream_t s, const float *Gt, double mean0 = 0.0);
+		float2 *spec, const float2 *twx, const float2 *twy, float *phi, cudaStream_t s, const float *Gt,
+		double mean0 = 0.0);
 } // namespace cpic

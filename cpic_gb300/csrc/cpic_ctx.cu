@@ -1419,13 +1419,13 @@ static int field_stage_async(cpic_ctx *c)
 			tot += (double) c->sp[s].n * (-c->sp[s].q / c->p.e0);
 		double mean0 = tot / ((double) c->g.nx * (double) c->g.ny);
 		CK(launch_poisson_mix(c->g, c->rho, c->qinv, nullptr, c->spec32, c->twx32, c->twy32,
-				c->cosx, c->cosy, c->phi32, st, c->green32, mean0));
+				c->phi32, st, c->green32, mean0));
 		launch_E_mix(c->g, c->phi32, c->E32, st);
 	}
 	else
 	{
 		CK(launch_poisson_f64(c->g, c->rho, c->qinv, c->spec64, c->twx64, c->twy64,
-				c->cosx, c->cosy, c->phi64, st, c->rho_lo, c->qinv_lo, c->green64));
+				c->phi64, st, c->rho_lo, c->qinv_lo, c->green64));
 		launch_E_f64(c->g, c->phi64, c->Ex64, c->Ey64, st);
 	}
 	CK(cudaGetLastError());

@@ -11,7 +11,10 @@ namespace cpic {
 // field_E_compute, src/field.c:358-416: E = -grad(phi) by central
 // differences, rows 0..ny (row ny is the south ghost), periodic through the
 // phi ghosts (src/comm_field.c:140-201), which equals periodic indexing.
-__global__ void k_E_f64(Grid g, const double *phi, double *Ex, double *Ey)
+// The divisions by 2 dx and 2 dy are bits::div_by (the quotient's value, three
+// FP64 instructions each: two divisions per node took 9 of the kernel's 12
+// us on a 512 x 512 grid).
+__global__ void k_E_f64(Grid g, const double *phi, double *Ex, double *Ey, double rdx2, double rdy2)
 {
 	double dx2 = 2 * g.dx, dy2 = 2 * g.dy;
 	// rows 0..ny over blockIdx.y (row ny is the south ghost: row 0 again)
@@ -26,8 +29,8 @@ __global__ void k_E_f64(Grid g, const double *phi, double *Ex, double *Ey)
 			int x0 = ix == 0 ? g.nx - 1 : ix - 1;
 			int x1 = ix + 1 == g.nx ? 0 : ix + 1;
 			int64_t i = (int64_t) iy * g.nx + ix;
-			Ey[i] = (phi[(int64_t) y0 * g.nx + ix] - phi[(int64_t) y1 * g.nx + ix]) / dy2;
-			Ex[i] = (phi[(int64_t) yc * g.nx + x0] - phi[(int64_t) yc * g.nx + x1]) / dx2;
+			Ey[i] = bits::div_by(phi[(int64_t) y0 * g.nx + ix] - phi[(int64_t) y1 * g.nx + ix], dy2, rdy2);
+			Ex[i] = bits::div_by(phi[(int64_t) yc * g.nx + x0] - phi[(int64_t) yc * g.nx + x1], dx2, rdx2);
 		}
 	}
 }
@@ -36,7 +39,7 @@ void launch_E_f64(const Grid &g, const double *phi, double *Ex, double *Ey, cuda
 {
 	dim3 grid((g.nx + 255) / 256, 1);
 	grid.y = (unsigned) std::min(g.ny + 1, std::max(1, 4096 / (int) grid.x));
-	k_E_f64<<<grid, 256, 0, s>>>(g, phi, Ex, Ey);
+	k_E_f64<<<grid, 256, 0, s>>>(g, phi, Ex, Ey, 1.0 / (2 * g.dx), 1.0 / (2 * g.dy));
 }
 
 // E at every particle (interpolate_f2p_E), written by particle id.  One
@@ -122,17 +125,15 @@ void launch_spill_f64(const SpillArgs &a, cudaStream_t s)
 }
 
 cudaError_t launch_poisson_f64(const Grid &g, const long long *rho, double qinv,
-		double2 *spec, const double2 *twx, const double2 *twy, const double *cosx,
-		const double *cosy, double *phi, cudaStream_t s, const long long *rho_lo, double qinv_lo,
-		const double *Gt)
+		double2 *spec, const double2 *twx, const double2 *twy, double *phi, cudaStream_t s,
+		const long long *rho_lo, double qinv_lo, const double *Gt)
 {
 	cudaError_t e = g_poisson_f64_once.run([] {
 		return set_max_dyn_smem({(const void *) k_rows_fwd<double>, (const void *) k_cols<double>,
-				(const void *) k_rows_inv<double>}, 200 * 1024);
+				(const void *) k_rows_inv<double>}, kFftMaxSmem);
 	});
 	if(e != cudaSuccess) return e;
-	poisson_launch<double>(g, rho, qinv, nullptr, spec, twx, twy, cosx, cosy, phi, s, rho_lo, qinv_lo,
-			Gt);
+	poisson_launch<double>(g, rho, qinv, nullptr, spec, twx, twy, phi, s, Gt, rho_lo, qinv_lo);
 	return cudaSuccess;
 }
 

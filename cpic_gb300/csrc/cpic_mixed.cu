@@ -221,16 +221,15 @@ void launch_spill_mix(const SpillArgs &a, cudaStream_t s)
 }
 
 cudaError_t launch_poisson_mix(const Grid &g, const long long *rho, double qinv, const long long *mean,
-		float2 *spec, const float2 *twx, const float2 *twy, const double *cosx,
-		const double *cosy, float *phi, cudaStream_t s, const float *Gt, double mean0)
+		float2 *spec, const float2 *twx, const float2 *twy, float *phi, cudaStream_t s, const float *Gt,
+		double mean0)
 {
 	cudaError_t e = g_poisson_mix_once.run([] {
 		return set_max_dyn_smem({(const void *) k_rows_fwd<float>, (const void *) k_cols<float>,
-				(const void *) k_rows_inv<float>}, 200 * 1024);
+				(const void *) k_rows_inv<float>}, kFftMaxSmem);
 	});
 	if(e != cudaSuccess) return e;
-	poisson_launch<float>(g, rho, qinv, mean, spec, twx, twy, cosx, cosy, phi, s, nullptr, 0.0, Gt,
-			mean0);
+	poisson_launch<float>(g, rho, qinv, mean, spec, twx, twy, phi, s, Gt, nullptr, 0.0, mean0);
 	return cudaSuccess;
 }
 

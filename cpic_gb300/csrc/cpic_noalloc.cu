@@ -6,9 +6,9 @@
 // cudaFree (which may synchronise the device) must not appear.  For them,
 // cpic_poisson_noalloc solves the same periodic Poisson problem as the
 // context's field stage (the MFT solve of the reference, solver.c:465-509)
-// with every piece of scratch -- the half spectrum, the FFT twiddles and the
-// Green's-function cosines -- in one file-scope __device__ array of fixed
-// size.  The caller passes its own input and output device buffers.
+// with every piece of scratch -- the half spectrum and the FFT twiddles, whose
+// real parts are the Green's-function cosines -- in one file-scope __device__
+// array of fixed size.  The caller passes its own input and output device buffers.
 //
 // The array is held by every GPU that loads this library until the process
 // exits (about 2.1 MB).  In host code the symbol is only a host-side
@@ -32,62 +32,66 @@ namespace {
 using namespace cpic;
 
 constexpr int kMaxN = CPIC_NOALLOC_MAX_N;            // nx, ny <= kMaxN
+constexpr int kLog2MaxN = 9;
+static_assert(1 << kLog2MaxN == kMaxN, "");
 constexpr size_t kSpecElems = (size_t) kMaxN * (kMaxN / 2 + 1);
-// layout: [spectrum kSpecElems double2][twx kMaxN/2 double2][twy kMaxN/2 double2]
-//         [cosx kMaxN double][cosy kMaxN double]
-constexpr size_t kScratchBytes = kSpecElems * sizeof(double2) + 2 * (kMaxN / 2) * sizeof(double2)
-	+ 2 * (size_t) kMaxN * sizeof(double);
+// layout: [spectrum kSpecElems double2][twiddles kMaxN/2 double2]
+constexpr size_t kScratchBytes = (kSpecElems + kMaxN / 2) * sizeof(double2);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
 constexpr int kMaxDevices = 64;
 static void *g_scratch_addr[kMaxDevices];
+static bool g_tables_ready[kMaxDevices];
 static std::mutex g_setup_lock;
 
-// Twiddles exp(-2 pi i k / n) and cosines cos(2 pi j / n), computed on the
-// device (sincospi: correctly scaled, ~1 ulp).
-__global__ void k_noalloc_tables(int nx, int ny, double2 *twx, double2 *twy, double *cosx,
-		double *cosy)
+// Twiddles exp(-2 pi i k / kMaxN), computed on the device (sincospi:
+// correctly scaled, ~1 ulp).  A transform of any smaller power of two reads
+// them with a stride, so one table, filled once per device, serves every
+// grid (filling tables of the call's own sizes took 9 us of every call).
+__global__ void k_noalloc_table(double2 *tw)
 {
-	for(int k = blockIdx.x * blockDim.x + threadIdx.x; k < kMaxN; k += gridDim.x * blockDim.x)
+	const int k = blockIdx.x * blockDim.x + threadIdx.x;
+	if(k < kMaxN / 2)
 	{
 		double s, c;
-		if(k < nx / 2) { sincospi(-2.0 * k / nx, &s, &c); twx[k] = make_double2(c, s); }
-		if(k < ny / 2) { sincospi(-2.0 * k / ny, &s, &c); twy[k] = make_double2(c, s); }
-		if(k < nx) cosx[k] = cospi(2.0 * k / nx);
-		if(k < ny) cosy[k] = cospi(2.0 * k / ny);
+		sincospi(-2.0 * k / kMaxN, &s, &c);
+		tw[k] = make_double2(c, s);
 	}
 }
 
-// rho (FP64, ny x nx) -> half spectra, two rows per block (the context's
-// rows_fwd reads fixed-point charge; this one reads the caller's doubles).
-__global__ void k_noalloc_rows_fwd(int nx, int log2nx, const double *rho, double2 *spec,
-		const double2 *tw)
+// cos(2 pi j / n), 0 <= j < n, from the table
+__device__ __forceinline__ double cos_of(const double2 *tw, int j, int log2n)
 {
-	extern __shared__ unsigned char smem_raw[];
-	double2 *a = reinterpret_cast<double2 *>(smem_raw);
-	double2 *b = a + nx;
-	int r0 = 2 * blockIdx.x;
-	int nh = nx / 2 + 1;
-	for(int i = threadIdx.x; i < nx; i += blockDim.x)
-		a[i] = make_double2(rho[(int64_t) r0 * nx + i], rho[(int64_t) (r0 + 1) * nx + i]);
-	__syncthreads();
-	double2 *Z = fft_smem<double2>(a, b, nx, log2nx, 1, -1, tw);
-	for(int k = threadIdx.x; k < nh; k += blockDim.x)
-	{
-		double2 p = Z[k], q = Z[(nx - k) & (nx - 1)];
-		q.y = -q.y;
-		spec[(int64_t) r0 * nh + k] = make_double2((p.x + q.x) * 0.5, (p.y + q.y) * 0.5);
-		spec[(int64_t) (r0 + 1) * nh + k] = make_double2((p.y - q.y) * 0.5, -(p.x - q.x) * 0.5);
-	}
+	const int m = j << (kLog2MaxN - log2n);
+	return m < kMaxN / 2 ? tw[m].x : -tw[m - kMaxN / 2].x;
+}
+
+// The columns with the Green's function evaluated here (no room for its
+// table): G(kx, ky) is even in ky, so each block divides for half of its
+// rows, into shared memory behind the transform's buffers.
+__global__ void k_noalloc_cols(const __grid_constant__ FftPlan py, int nh, int log2nx, double2 *spec,
+		const double2 *tw, size_t buf_bytes)
+{
+	extern __shared__ __align__(16) unsigned char smem_raw[];
+	double *gs = reinterpret_cast<double *>(smem_raw + buf_bytes);
+	const int kx = blockIdx.x, ny = py.n;
+	const double cx = cos_of(tw, kx, log2nx);
+	for(int row = threadIdx.x; row <= ny / 2; row += blockDim.x)
+		gs[row] = (kx == 0 && row == 0) ? 0.0 : 1.0 / (2.0 * (cx + cos_of(tw, row, py.log2n)) - 4.0);
+	cols_body<double>(py, nh, 1, spec, tw, kLog2MaxN - py.log2n, true, smem_raw,
+			[=](int, int row) { return gs[2 * row <= ny ? row : ny - row]; });
 }
 
 // Device address of the scratch array for the current device, looked up
 // once per device, together with the kernels' shared-memory limits (a
-// kernel attribute belongs to the device it was set on).  A device is marked
-// ready only when every step succeeded, so a failed set-up is retried by the
-// next call.
-static int scratch_for_current_device(void **out)
+// kernel attribute belongs to the device it was set on) and the twiddle
+// table, filled on the caller's stream: later calls are ordered behind it,
+// since calls that overlap on the GPU are the caller's to serialise.  A
+// device is marked ready only when every step succeeded, so a failed set-up
+// is retried by the next call; a table launch that was only recorded into a
+// graph does not count.
+static int scratch_for_current_device(void **out, cudaStream_t s)
 {
 	int dev = -1;
 	if(cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices)
@@ -99,13 +103,9 @@ static int scratch_for_current_device(void **out)
 		cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
 		if(e == cudaSuccess && !p)
 			e = cudaErrorInvalidSymbol;
-		// the largest blocks: two rows of kMaxN complex values, and the
-		// columns' two buffers of at most 128 KB together
 		if(e == cudaSuccess)
-			e = set_max_dyn_smem({(const void *) k_noalloc_rows_fwd,
-					(const void *) k_rows_inv<double>}, 2 * kMaxN * (int) sizeof(double2));
-		if(e == cudaSuccess)
-			e = set_max_dyn_smem({(const void *) k_cols<double>}, 128 * 1024);
+			e = set_max_dyn_smem({(const void *) k_rows_fwd_real<double>,
+					(const void *) k_noalloc_cols, (const void *) k_rows_inv<double>}, 64 * 1024);
 		if(e != cudaSuccess)
 		{
 			fprintf(stderr, "cpic_poisson_noalloc: set-up on device %d failed: %s\n", dev,
@@ -113,6 +113,23 @@ static int scratch_for_current_device(void **out)
 			return CPIC_ECUDA;
 		}
 		g_scratch_addr[dev] = p;
+	}
+	if(!g_tables_ready[dev])
+	{
+		cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+		double2 *tw = (double2 *) g_scratch_addr[dev] + kSpecElems;
+		void *argv[] = {&tw};
+		cudaError_t e = cudaLaunchKernel((const void *) k_noalloc_table, dim3(1), dim3(kMaxN / 2), argv,
+				0, s);
+		if(e == cudaSuccess)
+			e = cudaStreamIsCapturing(s, &cap);
+		if(e != cudaSuccess)
+		{
+			fprintf(stderr, "cpic_poisson_noalloc: set-up on device %d failed: %s\n", dev,
+					cudaGetErrorString(e));
+			return CPIC_ECUDA;
+		}
+		g_tables_ready[dev] = cap == cudaStreamCaptureStatusNone;
 	}
 	*out = g_scratch_addr[dev];
 	return CPIC_OK;
@@ -145,36 +162,25 @@ cpic_poisson_noalloc(const double *rho, double *phi, int64_t nx, int64_t ny, voi
 		return CPIC_EINVAL;
 	}
 	void *base = nullptr;
-	int r = scratch_for_current_device(&base);
-	if(r) return r;
 	cudaStream_t s = (cudaStream_t) stream;
-	unsigned char *p = (unsigned char *) base;
-	double2 *spec = (double2 *) p;
-	double2 *twx = (double2 *) (p + kSpecElems * sizeof(double2));
-	double2 *twy = twx + kMaxN / 2;
-	double *cosx = (double *) (twy + kMaxN / 2);
-	double *cosy = cosx + kMaxN;
-	int nxi = (int) nx, nyi = (int) ny;
-	int log2nx = 0, log2ny = 0;
-	while((1 << log2nx) < nxi) log2nx++;
-	while((1 << log2ny) < nyi) log2ny++;
+	int r = scratch_for_current_device(&base, s);
+	if(r) return r;
+	double2 *spec = (double2 *) base;
+	const double2 *tw = spec + kSpecElems;
+	const int nxi = (int) nx, nyi = (int) ny, nh = nxi / 2 + 1;
+	const FftPlan px = fft_plan(nxi), py = fft_plan(nyi);
+	const FftShape rs = fft_shape<double>(px, 1), cs = fft_shape<double>(py, 1);
+	const int sx = kLog2MaxN - px.log2n;
 
-	int rthreads = nxi / 2 < 32 ? 32 : (nxi / 2 > 512 ? 512 : nxi / 2);
-	int nh = nxi / 2 + 1;
-	int cb = (int) ((128 * 1024) / (2 * (size_t) nyi * sizeof(double2)));
-	if(cb < 1) cb = 1;
-	if(cb > nh) cb = nh;
-	const size_t rsm = 2 * (size_t) nxi * sizeof(double2);
-	const size_t csm = 2 * (size_t) cb * nyi * sizeof(double2);
-	cudaError_t e = launch(k_noalloc_tables, (kMaxN + 255) / 256, 256, 0, s, nxi, nyi, twx, twy,
-			cosx, cosy);
+	// one column per block, at most 257 of them
+	cudaError_t e = launch(k_rows_fwd_real<double>, nyi / 2, rs.threads, rs.smem, s, px, nyi, rho, spec,
+			tw, true, sx);
 	if(e == cudaSuccess)
-		e = launch(k_noalloc_rows_fwd, nyi / 2, rthreads, rsm, s, nxi, log2nx, rho, spec, twx);
+		e = launch(k_noalloc_cols, nh, cs.threads, cs.smem + (nyi / 2 + 1) * sizeof(double), s, py, nh,
+				px.log2n, spec, tw, cs.smem);
 	if(e == cudaSuccess)
-		e = launch(k_cols<double>, (nh + cb - 1) / cb, 512, csm, s, nxi, nyi, log2ny, cb, spec, twy,
-				cosx, cosy, nullptr);
-	if(e == cudaSuccess)
-		e = launch(k_rows_inv<double>, nyi / 2, rthreads, rsm, s, nxi, log2nx, nyi, spec, twx, phi);
+		e = launch(k_rows_inv<double>, nyi / 2, rs.threads, rs.smem, s, px, nyi, spec, tw, phi, true,
+				node_count<double>(nxi, nyi), sx);
 	if(e != cudaSuccess)
 	{
 		fprintf(stderr, "cpic_poisson_noalloc: launch failed: %s\n", cudaGetErrorString(e));
