@@ -50,7 +50,7 @@ int main()
 	for(int k = 0; k < 4000000; k++)
 		check_div(any(-300, 300), std::fabs(any(-40, 40)));
 	for(double d : {3.0, 0.1, 1e-3, 6.0e4})
-		for(double a : {0.0, INFINITY, -INFINITY, (double) NAN, 1.0, d, -d, 3 * d})
+		for(double a : {0.0, (double) INFINITY, (double) -INFINITY, (double) NAN, 1.0, d, -d, 3 * d})
 			check_div(a, d);
 	std::printf("%ld mismatches of %ld\n", bad, checked);
 	return bad != 0;
