@@ -30,7 +30,12 @@ namespace bits {
 CPIC_HD uint64_t to_bits(double d)
 {
 #ifdef __CUDA_ARCH__
-	return (uint64_t) __double_as_longlong(d);
+	// through an asm move: the compiler turns integer tests of a plain
+	// bit cast back into FP64 compares (four of them, 80 clocks of an SM per
+	// warp, in the fused kernel)
+	uint64_t b;
+	asm("mov.b64 %0, %1;" : "=l"(b) : "d"(d));
+	return b;
 #else
 	uint64_t b;
 	std::memcpy(&b, &d, 8);
@@ -96,6 +101,12 @@ CPIC_HD bool abs_gt(double d, double u)
 {
 	const uint64_t a = to_bits(d) & 0x7fffffffffffffffull;
 	return a > to_bits(u) && a <= 0x7ff0000000000000ull;
+}
+
+// d is +0.0 or -0.0
+CPIC_HD bool is_zero(double d)
+{
+	return (to_bits(d) << 1) == 0;
 }
 
 // d is neither infinite nor NaN
@@ -233,6 +244,203 @@ CPIC_HD bool split_fixed(double v, int lo_exp, long long &hi, long long &lo)
 	const bool lneg = neg != fneg;
 	hi = neg ? -(long long) him : (long long) him;
 	lo = lneg ? -(long long) lom : (long long) lom;
+	return true;
+}
+
+// ------------------------------------------------------------------------
+// FP64 arithmetic on the integer pipe.
+//
+// A positive normal double as its significand and exponent: (h:l) 2^(e - 63)
+// with bit 63 of the 64-bit h:l set and its low 11 bits zero.  The
+// operations below are IEEE 754's, rounded to nearest even, worked out on
+// these integers: the exact product or difference, then one rounding to 53
+// bits.  A product takes four 32 x 32 -> 64-bit multiplies and about 20
+// other instructions (7 clocks of an SM per warp), an FP64 multiply 20
+// clocks of its own pipe, which stays free for the rest of the particle's
+// arithmetic.  Operands that are zero, subnormal, negative or not finite are
+// not handled (false): the caller then uses the FP64 instructions.
+struct Pos {
+	uint32_t h, l;
+	int e;
+};
+
+CPIC_HD bool pos_of(double d, Pos &p)
+{
+	const uint64_t b = to_bits(d);
+	const uint32_t f = (uint32_t) (b >> 52);        // sign and exponent
+	p.h = (uint32_t) (b >> 21) | 0x80000000u;
+	p.l = (uint32_t) b << 11;
+	p.e = (int) f - 1023;
+	return f - 1u < 2046u;                  // positive, normal, finite
+}
+
+CPIC_HD uint64_t pos_bits(Pos p) { return (uint64_t) p.h << 32 | p.l; }
+
+// The double of p; its exponent must be that of a normal double (pos_normal).
+CPIC_HD double pos_val(Pos p)
+{
+	return from_bits((pos_bits(p) >> 11) + ((uint64_t) (uint32_t) (p.e + 1022) << 52));
+}
+
+CPIC_HD bool pos_normal(Pos p)
+{
+	return (uint32_t) (p.e + 1022) < 2046u;
+}
+
+// The upper word of (hi:lo) << n, n < 32.
+CPIC_HD uint32_t funnel_l(uint32_t lo, uint32_t hi, int n)
+{
+#ifdef __CUDA_ARCH__
+	return __funnelshift_l(lo, hi, n);
+#else
+	return n ? hi << n | lo >> (32 - n) : hi;
+#endif
+}
+
+CPIC_HD int clz32(uint32_t v)
+{
+#ifdef __CUDA_ARCH__
+	return __clz((int) v);
+#else
+	return v ? __builtin_clz(v) : 32;
+#endif
+}
+
+CPIC_HD int clz64(uint64_t v)
+{
+#ifdef __CUDA_ARCH__
+	return __clzll((long long) v);
+#else
+	return v ? __builtin_clzll(v) : 64;
+#endif
+}
+
+// h:l (bit 63 set), the bits below it by whether any is set, rounded to 53
+// bits: times 2^(e - 63).  The sum's bit 63 is clear only when it wrapped,
+// i.e. rounded up to the next power of two.
+CPIC_HD Pos pos_round(uint32_t h, uint32_t l, uint32_t below, int e)
+{
+	l |= below < 1u ? below : 1u;
+	const uint64_t t = ((uint64_t) h << 32 | l) + (0x3ffu + ((l >> 11) & 1u));
+	const uint32_t th = (uint32_t) (t >> 32);
+	Pos r;
+	r.h = th | 0x80000000u;
+	r.l = (uint32_t) t & ~0x7ffu;
+	r.e = e + 1 - (int) (th >> 31);
+	return r;
+}
+
+// The 128-bit product h:l1:l0 (h >= 2^62 as 64 bits) times 2^(e - 127),
+// rounded to 53 bits.
+CPIC_HD Pos pos_norm(uint64_t h, uint32_t l1, uint32_t l0, int e)
+{
+	const uint32_t hh = (uint32_t) (h >> 32), hl = (uint32_t) h;
+	const int n = (int) (hh >> 31) ^ 1;     // shift by one, or not
+	return pos_round(funnel_l(hl, hh, n), funnel_l(l1, hl, n), l1 << n | l0, e - n);
+}
+
+// rn(a b)
+CPIC_HD Pos pos_mul(Pos a, Pos b)
+{
+	const uint64_t p = (uint64_t) a.l * b.l;
+	const uint64_t t = (uint64_t) a.l * b.h + (uint32_t) (p >> 32);
+	const uint64_t u = (uint64_t) a.h * b.l + (uint32_t) t;
+	const uint64_t h = (uint64_t) a.h * b.h + (uint32_t) (t >> 32) + (uint32_t) (u >> 32);
+	return pos_norm(h, (uint32_t) u, (uint32_t) p, a.e + b.e + 1);
+}
+
+// rn(i b) for an integer i >= 1
+CPIC_HD Pos pos_mul_int(uint32_t i, Pos b)
+{
+	const int c = clz32(i);
+	const uint32_t a = i << c;
+	const uint64_t u = (uint64_t) a * b.l;
+	const uint64_t h = (uint64_t) a * b.h + (uint32_t) (u >> 32);
+	return pos_norm(h, (uint32_t) u, 0u, 32 - c + b.e);
+}
+
+// rn(1 - a) for 0 < a < 1 (a.e < 0)
+CPIC_HD Pos pos_one_minus(Pos a)
+{
+	if(a.e == -1)
+	{
+		// a >= 1/2: the difference is exact, in units of 2^-64
+		const uint64_t d = 0ull - pos_bits(a);
+		const int c = clz64(d);
+		const uint64_t m = d << c;
+		Pos r;
+		r.h = (uint32_t) (m >> 32);
+		r.l = (uint32_t) m;
+		r.e = -1 - c;
+		return r;
+	}
+	// a < 1/2: rounded to a multiple of 2^-53, 2^11 of the units.  x:
+	// 2^64 - floor(a 2^64), less one (an odd number, never a tie) when a bit
+	// of a lies below the units
+	const int sh = -1 - a.e;                // 1 ...
+	const uint64_t am = pos_bits(a);
+	const uint64_t q = sh < 64 ? am >> sh : 0ull;
+	const bool rest = sh >= 64 || (am << ((64 - sh) & 63)) != 0;
+	const uint64_t x = 0ull - (q | (rest ? 1ull : 0ull));
+	// (x == 0, a below the units with nothing left over, cannot happen: a
+	// shift of 64 or more leaves rest set)
+	return pos_round((uint32_t) (x >> 32), (uint32_t) x, 0u, -1);
+}
+
+// The cell index and the offset in the cell of position x > 0, as the FP64
+// sequence  i0 = floor(x idx);  rel = (x - i0 dx) idx  gives them; false
+// where a step is not handled (i0 out of range, an offset that is zero,
+// negative or 1 or more, a difference that would have to be rounded).
+CPIC_HD bool pos_rel(Pos x, Pos dx, Pos idx, int &i0, Pos &rel)
+{
+	const Pos p = pos_mul(x, idx);
+	if(p.e > 30)
+		return false;
+	uint32_t i = 0;
+	Pos d = x;                              // x - 0 dx
+	if(p.e >= 0)
+	{
+		i = p.h >> (31 - p.e);
+		const Pos s = pos_mul_int(i, dx);
+		const int k = x.e - s.e;
+		if((unsigned) (k + 1) > 2u)
+			return false;
+		// x is within a factor two of i dx: the difference is exact, in units
+		// of the smaller one's last place
+		const int kx = k > 0 ? 10 : 11, ks = k < 0 ? 10 : 11;
+		const int64_t v = (int64_t) (pos_bits(x) >> kx) - (int64_t) (pos_bits(s) >> ks);
+		if(v <= 0 || (v >> 53) != 0)
+			return false;
+		const int c = clz64((uint64_t) v);
+		const uint64_t m = (uint64_t) v << c;
+		d.h = (uint32_t) (m >> 32);
+		d.l = (uint32_t) m;
+		d.e = (k > 0 ? s.e : x.e) + 11 - c;
+	}
+	i0 = (int) i;
+	rel = pos_mul(d, idx);
+	return rel.e < 0;
+}
+
+// hi = rn(v), lo = rn((v - hi) 2^lo_exp), both negated when neg, as
+// split_fixed, for 1 <= v < 2^62 and 1 <= lo_exp <= 63 (false otherwise).
+CPIC_HD bool pos_split(Pos v, bool neg, int lo_exp, long long &hi, long long &lo)
+{
+	if((unsigned) v.e >= 62u)
+		return false;
+	const int sh = 63 - v.e;                // 2 .. 63 fractional bits of m
+	const uint64_t m = pos_bits(v);
+	const uint64_t q = m >> sh;
+	const uint64_t r = m << (64 - sh);      // the fraction, in units of 2^-64
+	// up past one half, or at it from an odd integer
+	const bool up = r > (1ull << 63) - (q & 1ull);
+	const uint64_t f = up ? 0ull - r : r;   // |v - hi|
+	const uint64_t g = f >> (64 - lo_exp);
+	const uint64_t rem = f << lo_exp;
+	const bool up2 = rem > (1ull << 63) - (g & 1ull);
+	const uint64_t h = q + (up ? 1ull : 0ull), l = g + (up2 ? 1ull : 0ull);
+	hi = neg ? -(long long) h : (long long) h;
+	lo = neg != up ? -(long long) l : (long long) l;
 	return true;
 }
 

@@ -129,6 +129,10 @@ struct SpeciesStep {
 	double qfix;         // fixed-point units per unit of w: -q/e0 * qscale
 	double qlo_mul;      // FP64 form: 2^m, the scale of the remainder word
 	int qlo_exp;         // m
+	// FP64 form: |qfix| and its sign for the integer path of the push, which
+	// runs when fast is set (every constant it needs a normal double)
+	bits::Pos qfix_p;
+	int qfix_neg, fast;
 	double wq_scale;     // mixed: fixed-point units per integer weight unit
 	long long wq_int;    // the same as an integer when it is one, else 0
 	float dtqm2_f, tz_f, sz_f;
@@ -147,6 +151,7 @@ struct PushArgs {
 	int arr_r;           // arrivals buffer read by this step (movers go to 1 - arr_r)
 	int iter;            // 0 -> backward half step, no move
 	double dt;
+	bits::Pos dx_p, idx_p, idy_p;  // g.dx, g.idx, g.idy (FP64 form)
 	float cdx_f, cdy_f;  // dt/dx, dt/dy (mixed form)
 	SpeciesStep sp[kMaxSpecies];
 	Tiles tiles[kMaxSpecies];
@@ -274,6 +279,18 @@ dep_global2(long long *rho, long long *rlo, const Grid &g, int cx, int cy,
 		red_global(&rho[n[c]], hi[c]);
 		red_global(&rlo[n[c]], lo[c]);
 	}
+}
+
+// Adds v to a 64-bit sum kept as two 32-bit words in shared memory: the low
+// word's atomic returns its old value, whose carry goes into the high word's,
+// so the sum is exact modulo 2^64 whatever the order of the additions.
+// Shared memory has native 32-bit atomic additions only; a 64-bit one is a
+// compare-and-swap loop.
+__device__ __forceinline__ uint32_t add64_low(uint32_t *lo, long long v)
+{
+	const uint32_t x = (uint32_t) v;
+	const uint32_t old = atomicAdd(lo, x);
+	return (uint32_t) ((uint64_t) v >> 32) + (old > ~x ? 1u : 0u);
 }
 
 // Global node index of shared accumulator entry i (frame origin t0 - H).

@@ -855,6 +855,8 @@ static void fill_species_step(cpic_ctx *c, PushArgs &a, int64_t iter)
 	a.cdx_f = (float) (p.dt / c->g.dx);
 	a.cdy_f = (float) (p.dt / c->g.dy);
 	int64_t chunks = p.plasma_chunks > 0 ? p.plasma_chunks : 1;
+	const bool consts = bits::pos_of(c->g.dx, a.dx_p) & bits::pos_of(c->g.idx, a.idx_p)
+		& bits::pos_of(c->g.idy, a.idy_p);
 	for(int s = 0; s < c->nspecies; s++)
 	{
 		SpeciesStep &st = a.sp[s];
@@ -873,6 +875,9 @@ static void fill_species_step(cpic_ctx *c, PushArgs &a, int64_t iter)
 		st.qfix = vq * c->qscale;
 		st.qlo_mul = c->qlo_mul;
 		st.qlo_exp = ilogb(c->qlo_mul);
+		st.qfix_neg = st.qfix < 0.0;
+		st.fast = bits::pos_of(fabs(st.qfix), st.qfix_p) && st.qlo_exp >= 1 && st.qlo_exp <= 63
+			&& consts;
 		st.wq_scale = c->wq_exact ? c->sp[s].wq_mult : st.qfix * ldexp(1.0, -kWeightBits);
 		st.wq_int = c->wq_exact ? (long long) c->sp[s].wq_mult : 0;
 		st.dtqm2_f = (float) st.dtqm2;
@@ -1743,21 +1748,23 @@ CPIC_API int cpic_add_species(cpic_ctx_t *c, double q, double m, int64_t n,
 	memset((void *) &S, 0, sizeof(S));
 	S.q = q; S.m = m; S.n = n;
 	S.vmax = vmax;
-	// the fused kernel's instance when the caller left it to the library:
-	// 1 particle per thread (chunks of 256) while every species has fewer
-	// than kSmallTile particles per tile, else 2 (chunks of 512).  A tile's
-	// last main-region chunk and its arrivals chunk are partial, and on
-	// small tiles they and the latency between chunks dominate: the FP64
-	// two-species 512x512 workload (about 1,100 particles per 8x8 tile and
-	// species) steps in 1.498 ms with 1, 1.678 ms with 2; two-stream 2048x2048
-	// (102,400 per tile) is fastest with 2.
+	// the fused kernel's instance when the caller left it to the library.
+	// FP64: 1 particle per thread; the kernel's arithmetic is long enough to
+	// hide a chunk's latency, and a second copy of its code misses the
+	// instruction cache (two-stream 512x512, 100 per cell: 1911 us per launch
+	// with 1, 2503 with 2; two species, 16 per cell: 357 and 470).
+	// Mixed: 1 while every species has fewer than kSmallTile particles per
+	// tile, else 2 (chunks of 512).  A tile's last main-region chunk and its
+	// arrivals chunk are partial, and on small tiles they and the latency
+	// between chunks dominate; two-stream 2048x2048 (102,400 per tile) is
+	// fastest with 2.
 	if(c->p.particles_per_thread <= 0)
 	{
 		constexpr int64_t kSmallTile = 4096;
 		bool small = n / std::max(1, c->ntiles) < kSmallTile;
 		for(int k = 0; k < c->nspecies; k++)
 			small = small && c->sp[k].n / std::max(1, c->ntiles) < kSmallTile;
-		c->ppt = small ? 1 : kPPT;
+		c->ppt = small || c->precision == CPIC_FP64 ? 1 : kPPT;
 	}
 	int nt = c->ntiles;
 	CK(cudaMalloc(&S.tiles.base, nt * sizeof(int64_t)));

@@ -80,9 +80,9 @@ static const void *push_f64_fn(int P)
 {
 	switch(P)
 	{
-		case 1: return (const void *) k_push<F64, F64::kMinBlocks, true, 1>;
-		case 4: return (const void *) k_push<F64, F64::kMinBlocks, true, 4>;
-		default: return (const void *) k_push<F64, F64::kMinBlocks, true, 2>;
+		case 1: return (const void *) k_push<F64, F64::min_blocks(1), true, 1>;
+		case 4: return (const void *) k_push<F64, F64::min_blocks(4), true, 4>;
+		default: return (const void *) k_push<F64, F64::min_blocks(2), true, 2>;
 	}
 }
 
@@ -112,9 +112,9 @@ cudaError_t launch_push_f64(const PushArgs &a, int ntiles, size_t smem, int ppt,
 	for(int sp = 0; sp < a.nspecies; sp++)
 	{
 		const PushArgs b = species_args(a, sp);
-		if(ppt == 1) k_push<F64, F64::kMinBlocks, true, 1><<<ntiles, kPushThreads, smem, s>>>(b);
-		else if(ppt == 4) k_push<F64, F64::kMinBlocks, true, 4><<<ntiles, kPushThreads, smem, s>>>(b);
-		else k_push<F64, F64::kMinBlocks, true, 2><<<ntiles, kPushThreads, smem, s>>>(b);
+		if(ppt == 1) k_push<F64, F64::min_blocks(1), true, 1><<<ntiles, kPushThreads, smem, s>>>(b);
+		else if(ppt == 4) k_push<F64, F64::min_blocks(4), true, 4><<<ntiles, kPushThreads, smem, s>>>(b);
+		else k_push<F64, F64::min_blocks(2), true, 2><<<ntiles, kPushThreads, smem, s>>>(b);
 	}
 	return cudaSuccess;
 }

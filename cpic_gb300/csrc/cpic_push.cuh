@@ -35,7 +35,13 @@ namespace cpic {
 
 struct F64 {
 	struct Rec { double x, y, ux, uy; int32_t id; };
-	static constexpr int kMinBlocks = 1;
+	// Resident blocks per SM the registers are capped for, by particles per
+	// thread: the integer arithmetic is latency bound, and more warps pay for
+	// the few spills (one particle per thread, two-stream 512 x 512 with 100
+	// per cell: 2262 us per launch uncapped with 3 blocks, 2222 with 4; after
+	// the pass loop below 1947 with 4, 1911 with 5).
+	static constexpr int min_blocks(int P) { return P == 1 ? kMinBlocks : P == 2 ? 4 : 2; }
+	static constexpr int kMinBlocks = 5;
 
 	struct Out {
 		int dest;        // destination tile
@@ -47,7 +53,9 @@ struct F64 {
 		uint32_t err;
 	};
 
-	// shared memory: W x W 64-bit high words, then W x W remainder words
+	// shared memory: the W x W 64-bit sums and their remainder words as four
+	// planes of 32-bit words (add64_low): low and high half of the sums, low
+	// and high half of the remainders
 	static __host__ __device__ size_t smem_bytes(int W, int T)
 	{
 		return 2 * (size_t) W * W * sizeof(long long);
@@ -167,8 +175,67 @@ struct F64 {
 		ey = v;
 	}
 
+	// The cell of (x, y) and its four CIC weights on the integer pipe
+	// (cpic_bits.h: the values weights() gives); false where a step of it is
+	// not handled there.
+	static __device__ __forceinline__ bool weights_fast(const PushArgs &a, double x, double y,
+			bits::Pos w[4], int &i0x, int &i0y)
+	{
+		bits::Pos px, py, rx, ry;
+		bool ok = bits::pos_of(x, px) & bits::pos_of(y, py);
+		ok = ok && bits::pos_rel(px, a.dx_p, a.idx_p, i0x, rx)
+			&& bits::pos_rel(py, a.dx_p, a.idy_p, i0y, ry);
+		if(!ok)
+			return false;
+		const bits::Pos dx = bits::pos_one_minus(rx), dy = bits::pos_one_minus(ry);
+		w[0] = bits::pos_mul(dx, dy);
+		w[1] = bits::pos_mul(dx, ry);
+		w[2] = bits::pos_mul(rx, dy);
+		w[3] = bits::pos_mul(rx, ry);
+		return true;
+	}
+
+	// The same on FP64 instructions, out of line: rarely taken, and the
+	// kernel's code is already larger than the instruction caches like.
+	struct SlowWeights { double w[4]; int i0x, i0y; };
+	static __device__ __noinline__ SlowWeights weights_slow(const PushArgs &a, double x, double y)
+	{
+		SlowWeights d;
+		weights(a.g, x, y, d.w, d.i0x, d.i0y);
+		return d;
+	}
+
+	struct SlowDeposit { long long hi[4], lo[4]; int i0x, i0y; };
+	static __device__ __noinline__ SlowDeposit deposit_slow(const PushArgs &a, const SpeciesStep &sp,
+			double x, double y)
+	{
+		SlowDeposit d;
+		double w[4];
+		weights(a.g, x, y, w, d.i0x, d.i0y);
+		for(int c = 0; c < 4; c++)
+		{
+			double v = w[c] * sp.qfix;
+			// the split on the integer pipe (cpic_bits.h: exact, the same
+			// values), the FP64 instructions for what it does not take
+			if(!bits::split_fixed(v, sp.qlo_exp, d.hi[c], d.lo[c]))
+			{
+				d.hi[c] = __double2ll_rn(v);
+				d.lo[c] = __double2ll_rn((v - (double) d.hi[c]) * sp.qlo_mul);
+			}
+		}
+		return d;
+	}
+
 	// One particle.  tx0/ty0: origin of the tile it is processed in.
 	// deposit_only: keep the state, only compute the deposit (pre-step).
+	//
+	// The FP64 pipe bounds this kernel (20 clocks of an SM per warp
+	// instruction; 70 of them for the arithmetic as written).  The weights of
+	// the old and the new position and the fixed-point deposit values are
+	// therefore computed on integers (weights_fast, pos_mul, pos_split: the
+	// same values, bit for bit), which leaves the FP64 pipe the gather, the
+	// kick and the move; positions the integer path does not take (on a cell
+	// edge, in the box's corner cells next to 0) use the FP64 instructions.
 	template <bool GP2 = true>
 	static __device__ __forceinline__ Out push(const PushArgs &a, int s, Rec &r,
 			int tx0, int ty0, const void *)
@@ -178,79 +245,100 @@ struct F64 {
 		Out o;
 		o.err = 0;
 		o.quirk = 0;
-		double w[4];
 		int i0x, i0y;
-		weights(g, r.x, r.y, w, i0x, i0y);
-		if(i0x < 0 || i0y < 0 || i0x > g.nx || i0y > g.ny)
-		{
-			o.err |= ST_RANGE;
-			i0x = min(max(i0x, 0), g.nx - 1);
-			i0y = min(max(i0y, 0), g.ny - 1);
-		}
-		double ex, ey;
-		gather(a.Ex64, a.Ey64, g, w, i0x, i0y, ex, ey);
-
-		// boris_rotation, mover.c:22-70, with B = (0, 0, Bz): the terms
-		// multiplied by the exact zeros t[X], t[Y], s[X], s[Y] vanish
-		// exactly, leaving these operations in the same order.
-		double dtqm2 = sp.dtqm2;
-		double vmx = r.ux + dtqm2 * ex;
-		double vmy = r.uy + dtqm2 * ey;
-		double vpx = vmy * sp.tz + vmx;
-		double vpy = vmy - vmx * sp.tz;
-		double vlx = vpy * sp.sz + vmx;
-		double vly = vmy - vpx * sp.sz;
-		double ux = vlx + dtqm2 * ex;
-		double uy = vly + dtqm2 * ey;
-
-		// check_velocity, mover.c:97-137 (the compares on the integer
-		// pipe, cpic_bits.h: the same results)
-		if(bits::abs_gt(ux, sp.umax_x) || bits::abs_gt(uy, sp.umax_y))
-			o.err |= ST_UMAX;
-		if(!bits::is_finite(ux) || !bits::is_finite(uy))
-			o.err |= ST_NAN;
-
 		double x = r.x, y = r.y;
-		if(a.iter != 0)
+		// pass 0: the weights of the old position, gather, kick and move;
+		// pass 1: those of the new position, the deposit values.  A loop, not
+		// two copies: the weights' code is half of the kernel, which misses
+		// the instruction cache as it is.
+		#pragma unroll 1
+		for(int pass = 0; ; pass++)
 		{
-			// move, mover.c:74-82
-			x += ux * a.dt;
-			y += uy * a.dt;
-		}
-		// periodic_boundary_ppack, comm_plasma.c:725-747 (X then Y; the
-		// compares on the integer pipe, cpic_bits.h).  A branch around the
-		// rare wrap: computed for every particle and selected, the two
-		// additions took 4 % of the FP64 form's time.
-		if(__builtin_expect(bits::ge_pos(x, g.Lx) || bits::lt_zero(x), 0))
-			x = bits::ge_pos(x, g.Lx) ? x - g.Lx : x + g.Lx;
-		if(__builtin_expect(bits::ge_pos(y, g.Ly) || bits::lt_zero(y), 0))
-			y = bits::ge_pos(y, g.Ly) ? y - g.Ly : y + g.Ly;
-		if(!bits::is_finite(x) || !bits::is_finite(y))
-		{
-			o.err |= ST_NAN;
-			x = 0.0; y = 0.0;
-		}
-		r.x = x; r.y = y; r.ux = ux; r.uy = uy;
-
-		// deposit weights of the new position (interpolate_p2f,
-		// interpolate.c:161-276), value w * (-q/e0) in two-word fixed
-		// point: c = w * qfix is the reference's addend scaled by 2^k
-		// (exactly: a power-of-two scale), hi its rounding, and the
-		// remainder c - hi (exact) is kept at 2^m finer resolution.
-		weights(g, x, y, w, i0x, i0y);
-		for(int c = 0; c < 4; c++)
-		{
-			double v = w[c] * sp.qfix;
-			// the split on the integer pipe (cpic_bits.h: exact, the same
-			// values), the FP64 instructions for what it does not take
-			long long hi, lo;
-			if(!bits::split_fixed(v, sp.qlo_exp, hi, lo))
+			bits::Pos wp[4];
+			bool fast = sp.fast && weights_fast(a, x, y, wp, i0x, i0y);
+			if(pass)
 			{
-				hi = __double2ll_rn(v);
-				lo = __double2ll_rn((v - (double) hi) * sp.qlo_mul);
+				// deposit weights of the new position (interpolate_p2f,
+				// interpolate.c:161-276), value w * (-q/e0) in two-word fixed
+				// point: c = w * qfix is the reference's addend scaled by 2^k
+				// (exactly: a power-of-two scale), hi its rounding, and the
+				// remainder c - hi (exact) is kept at 2^m finer resolution.
+				for(int c = 0; c < 4; c++)
+					fast = fast && bits::pos_split(bits::pos_mul(wp[c], sp.qfix_p), sp.qfix_neg != 0,
+							sp.qlo_exp, o.w[c], o.wl[c]);
+				if(!fast)
+				{
+					const SlowDeposit d = deposit_slow(a, sp, x, y);
+					i0x = d.i0x; i0y = d.i0y;
+					for(int c = 0; c < 4; c++) { o.w[c] = d.hi[c]; o.wl[c] = d.lo[c]; }
+				}
+				break;
 			}
-			o.w[c] = hi;
-			o.wl[c] = lo;
+			double w[4];
+			fast = fast && bits::pos_normal(wp[0]) && bits::pos_normal(wp[1])
+				&& bits::pos_normal(wp[2]) && bits::pos_normal(wp[3]);
+			if(fast)
+				for(int c = 0; c < 4; c++) w[c] = bits::pos_val(wp[c]);
+			else
+			{
+				const SlowWeights d = weights_slow(a, x, y);
+				i0x = d.i0x; i0y = d.i0y;
+				for(int c = 0; c < 4; c++) w[c] = d.w[c];
+			}
+			if(i0x < 0 || i0y < 0 || i0x > g.nx || i0y > g.ny)
+			{
+				o.err |= ST_RANGE;
+				i0x = min(max(i0x, 0), g.nx - 1);
+				i0y = min(max(i0y, 0), g.ny - 1);
+			}
+			double ex, ey;
+			gather(a.Ex64, a.Ey64, g, w, i0x, i0y, ex, ey);
+
+			// boris_rotation, mover.c:22-70, with B = (0, 0, Bz): the terms
+			// multiplied by the exact zeros t[X], t[Y], s[X], s[Y] vanish
+			// exactly, leaving these operations in the same order.
+			double dtqm2 = sp.dtqm2;
+			double vmx = r.ux + dtqm2 * ex;
+			double vmy = r.uy + dtqm2 * ey;
+			double vlx = vmx, vly = vmy;
+			if(!bits::is_zero(sp.tz))
+			{
+				// (without a field the rotation adds zeros: the same values)
+				double vpx = vmy * sp.tz + vmx;
+				double vpy = vmy - vmx * sp.tz;
+				vlx = vpy * sp.sz + vmx;
+				vly = vmy - vpx * sp.sz;
+			}
+			double ux = vlx + dtqm2 * ex;
+			double uy = vly + dtqm2 * ey;
+
+			// check_velocity, mover.c:97-137 (the compares on the integer
+			// pipe, cpic_bits.h: the same results)
+			if(bits::abs_gt(ux, sp.umax_x) || bits::abs_gt(uy, sp.umax_y))
+				o.err |= ST_UMAX;
+			if(!bits::is_finite(ux) || !bits::is_finite(uy))
+				o.err |= ST_NAN;
+
+			if(a.iter != 0)
+			{
+				// move, mover.c:74-82
+				x += ux * a.dt;
+				y += uy * a.dt;
+			}
+			// periodic_boundary_ppack, comm_plasma.c:725-747 (X then Y; the
+			// compares on the integer pipe, cpic_bits.h).  A branch around the
+			// rare wrap: computed for every particle and selected, the two
+			// additions took 4 % of the FP64 form's time.
+			if(__builtin_expect(bits::ge_pos(x, g.Lx) || bits::lt_zero(x), 0))
+				x = bits::ge_pos(x, g.Lx) ? x - g.Lx : x + g.Lx;
+			if(__builtin_expect(bits::ge_pos(y, g.Ly) || bits::lt_zero(y), 0))
+				y = bits::ge_pos(y, g.Ly) ? y - g.Ly : y + g.Ly;
+			if(!bits::is_finite(x) || !bits::is_finite(y))
+			{
+				o.err |= ST_NAN;
+				x = 0.0; y = 0.0;
+			}
+			r.x = x; r.y = y; r.ux = ux; r.uy = uy;
 		}
 		if(i0x >= g.nx || i0y >= g.ny || i0x < 0 || i0y < 0)
 		{
@@ -276,8 +364,8 @@ struct F64 {
 
 	static __device__ __forceinline__ void clear(unsigned char *sm, int W, int T)
 	{
-		long long *acc = reinterpret_cast<long long *>(sm);
-		for(int i = threadIdx.x; i < 2 * W * W; i += blockDim.x)
+		uint32_t *acc = reinterpret_cast<uint32_t *>(sm);
+		for(int i = threadIdx.x; i < 4 * W * W; i += blockDim.x)
 			acc[i] = 0;
 	}
 
@@ -313,16 +401,22 @@ struct F64 {
 		int lx = o.rx + H, ly = o.ry + H;
 		if(sm && (unsigned) lx < (unsigned) (W - 1) && (unsigned) ly < (unsigned) (W - 1))
 		{
-			long long *p = reinterpret_cast<long long *>(sm) + ly * W + lx;
-			long long *q = p + W * W;
-			atomicAdd((unsigned long long *) &p[0], (unsigned long long) o.w[0]);
-			atomicAdd((unsigned long long *) &p[W], (unsigned long long) o.w[1]);
-			atomicAdd((unsigned long long *) &p[1], (unsigned long long) o.w[2]);
-			atomicAdd((unsigned long long *) &p[W + 1], (unsigned long long) o.w[3]);
-			atomicAdd((unsigned long long *) &q[0], (unsigned long long) o.wl[0]);
-			atomicAdd((unsigned long long *) &q[W], (unsigned long long) o.wl[1]);
-			atomicAdd((unsigned long long *) &q[1], (unsigned long long) o.wl[2]);
-			atomicAdd((unsigned long long *) &q[W + 1], (unsigned long long) o.wl[3]);
+			const int pl = W * W;
+			uint32_t *p = reinterpret_cast<uint32_t *>(sm) + ly * W + lx;
+			const int at[4] = {0, W, 1, W + 1};
+			// every low word first: the additions that wait for a carry then
+			// overlap
+			uint32_t h[4], hl[4];
+			for(int c = 0; c < 4; c++)
+			{
+				h[c] = add64_low(p + at[c], o.w[c]);
+				hl[c] = add64_low(p + at[c] + 2 * pl, o.wl[c]);
+			}
+			for(int c = 0; c < 4; c++)
+			{
+				atomicAdd(p + at[c] + pl, h[c]);
+				atomicAdd(p + at[c] + 3 * pl, hl[c]);
+			}
 		}
 		else
 			dep_global2(a.rho, a.rho_lo, g, tx0 + o.rx, ty0 + o.ry, o.w, o.wl);
@@ -331,10 +425,12 @@ struct F64 {
 	static __device__ __forceinline__ void flush(const PushArgs &a, int s, unsigned char *sm,
 			int W, int H, int tx0, int ty0)
 	{
-		const long long *acc = reinterpret_cast<const long long *>(sm);
-		for(int i = threadIdx.x; i < W * W; i += blockDim.x)
+		const uint32_t *acc = reinterpret_cast<const uint32_t *>(sm);
+		const int pl = W * W;
+		for(int i = threadIdx.x; i < pl; i += blockDim.x)
 		{
-			long long v = acc[i], vl = acc[W * W + i];
+			const long long v = (long long) ((uint64_t) acc[pl + i] << 32 | acc[i]);
+			const long long vl = (long long) ((uint64_t) acc[3 * pl + i] << 32 | acc[2 * pl + i]);
 			int64_t node = frame_node(a.g, W, H, tx0, ty0, i);
 			if(v != 0) red_global(&a.rho[node], v);
 			if(vl != 0) red_global(&a.rho_lo[node], vl);

@@ -67,8 +67,9 @@ typedef struct cpic_params {
 	int32_t halo;            /* deposit halo in cells; 0 = auto */
 	int32_t track_ids;       /* keep a particle id per particle (MIXED) */
 	int32_t particles_per_thread; /* fused kernel instance: 1, 2 or 4; 0 = chosen
-	                               * at cpic_add_species: 1 while every species
-	                               * has < 4096 particles per tile, else 2 */
+	                               * at cpic_add_species: FP64 1; mixed 1 while
+	                               * every species has < 4096 particles per
+	                               * tile, else 2 */
 	int32_t reserved[6];
 } cpic_params_t;
 
