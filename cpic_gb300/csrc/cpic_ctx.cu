@@ -143,7 +143,8 @@ constexpr int kOrderKeys = 512;
 constexpr int kOrderMid = kOrderKeys - 1 - 255;      // bucket of the middle class
 constexpr int kOrderThreads = 1024;
 constexpr int kOrderMaxTiles = 8192;                 // larger layouts keep tile order
-constexpr int kOrderPer = kOrderMaxTiles / kOrderThreads;
+constexpr int kOrderPer = kOrderMaxTiles / kOrderThreads;   // per thread, and 32-tile rounds per warp
+static_assert(kOrderMaxTiles <= 65535 && kOrderKeys <= kOrderThreads, "16-bit places, a thread per bucket");
 
 __device__ __forceinline__ int order_bucket(int32_t cnt, int ntiles, long long sum)
 {
@@ -160,46 +161,51 @@ __device__ __forceinline__ int order_bucket(int32_t cnt, int ntiles, long long s
 
 // One block of kOrderThreads per species: the counts are read once, in
 // parallel; a uniform layout (every tile in the middle class) writes the
-// identity at once; otherwise warp 0 scans the bucket counts and scatters
-// from the buckets kept in shared memory.
+// identity at once.  Otherwise every warp ranks the tiles of a contiguous
+// range among those of their bucket before them in the range (its own
+// counters, so tile order is kept without atomics), a scan over buckets and
+// warps gives each warp's first place in each bucket, and all tiles are
+// placed at once.  (One warp scattering alone took 23 us for 4096 tiles,
+// more than a small run's field solve.)
 __global__ void __launch_bounds__(kOrderThreads) k_tile_order(const PushArgs a, int ntiles, int abuf)
 {
+	constexpr int kWarps = kOrderThreads / 32;
 	const Tiles &T = a.tiles[blockIdx.x];
-	__shared__ uint16_t s_b[kOrderMaxTiles];
-	__shared__ int32_t cur[kOrderKeys];
-	__shared__ long long s_part[kOrderThreads / 32];
+	__shared__ uint16_t s_cnt[kWarps][kOrderKeys];   // then: first place
+	__shared__ int32_t s_wsum[kWarps];
+	__shared__ long long s_part[kWarps];
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	// warp w takes tiles [w per, (w + 1) per), 32 at a time
+	const int per = (ntiles + kOrderThreads - 1) / kOrderThreads * 32;
+	const int first = warp * per;
 	int32_t c[kOrderPer];
 	long long sum = 0;
 	#pragma unroll
 	for(int k = 0; k < kOrderPer; k++)
 	{
-		const int i = k * kOrderThreads + tid;
-		c[k] = i < ntiles ? T.cnt[i] + T.acnt[abuf][i] : 0;
+		const int i = first + k * 32 + lane;
+		c[k] = k * 32 < per && i < ntiles ? T.cnt[i] + T.acnt[abuf][i] : 0;
 		sum += c[k];
 	}
 	for(int o = 16; o > 0; o >>= 1)
 		sum += __shfl_xor_sync(0xffffffffu, sum, o);
 	if(lane == 0)
 		s_part[warp] = sum;
-	for(int k = tid; k < kOrderKeys; k += kOrderThreads)
-		cur[k] = 0;
+	for(int k = tid; k < kWarps * kOrderKeys; k += kOrderThreads)
+		(&s_cnt[0][0])[k] = 0;
 	__syncthreads();
 	sum = 0;
-	for(int w = 0; w < kOrderThreads / 32; w++)
+	for(int w = 0; w < kWarps; w++)
 		sum += s_part[w];
 	int moved = 0;
+	int b[kOrderPer];
 	#pragma unroll
 	for(int k = 0; k < kOrderPer; k++)
 	{
-		const int i = k * kOrderThreads + tid;
-		if(i < ntiles)
-		{
-			const int b = sum > 0 ? order_bucket(c[k], ntiles, sum) : kOrderMid;
-			s_b[i] = (uint16_t) b;
-			moved |= b != kOrderMid;
-			atomicAdd(&cur[b], 1);
-		}
+		const int i = first + k * 32 + lane;
+		const bool on = k * 32 < per && i < ntiles;
+		b[k] = on ? (sum > 0 ? order_bucket(c[k], ntiles, sum) : kOrderMid) : -1;
+		moved |= on && b[k] != kOrderMid;
 	}
 	if(!__syncthreads_or(moved))
 	{
@@ -207,46 +213,56 @@ __global__ void __launch_bounds__(kOrderThreads) k_tile_order(const PushArgs a, 
 			T.order[i] = i;
 		return;
 	}
-	if(warp != 0)
-		return;
-	// exclusive scan: lane l owns buckets [16 l, 16 l + 16)
-	constexpr int per = kOrderKeys / 32;
-	int loc = 0;
-	for(int k = 0; k < per; k++)
-		loc += cur[lane * per + k];
-	int inc = loc;
+	int rank[kOrderPer];
+	#pragma unroll
+	for(int k = 0; k < kOrderPer; k++)
+	{
+		const unsigned peers = __match_any_sync(0xffffffffu, b[k]);
+		const int before = __popc(peers & lanemask_lt());
+		rank[k] = b[k] >= 0 ? s_cnt[warp][b[k]] + before : 0;
+		__syncwarp();
+		if(b[k] >= 0 && before == 0)
+			s_cnt[warp][b[k]] += (uint16_t) __popc(peers);
+		__syncwarp();
+	}
+	__syncthreads();
+	// thread t < kOrderKeys: bucket t over the warps, then over the buckets
+	int total = 0;
+	if(tid < kOrderKeys)
+		for(int w = 0; w < kWarps; w++)
+		{
+			const int n = s_cnt[w][tid];
+			s_cnt[w][tid] = (uint16_t) total;
+			total += n;
+		}
+	int inc = total;
 	for(int o = 1; o < 32; o <<= 1)
 	{
-		int v = __shfl_up_sync(0xffffffffu, inc, o);
+		const int v = __shfl_up_sync(0xffffffffu, inc, o);
 		if(lane >= o) inc += v;
 	}
-	int run = inc - loc;
-	for(int k = 0; k < per; k++)
+	if(lane == 31)
+		s_wsum[warp] = inc;
+	__syncthreads();
+	if(tid < kOrderKeys)
 	{
-		int v = cur[lane * per + k];
-		cur[lane * per + k] = run;
-		run += v;
+		int base = inc - total;
+		for(int w = 0; w < warp; w++)
+			base += s_wsum[w];
+		for(int w = 0; w < kWarps; w++)
+			s_cnt[w][tid] = (uint16_t) (s_cnt[w][tid] + base);
 	}
-	__syncwarp();
-	// stable scatter, 32 tiles at a time in tile order
-	for(int i0 = 0; i0 < ntiles; i0 += 32)
-	{
-		const int i = i0 + lane;
-		const int b = i < ntiles ? (int) s_b[i] : -1;
-		const unsigned peers = __match_any_sync(0xffffffffu, b);
-		const int pos = b >= 0 ? cur[b] + __popc(peers & lanemask_lt()) : 0;
-		__syncwarp();
-		if(b >= 0)
+	__syncthreads();
+	#pragma unroll
+	for(int k = 0; k < kOrderPer; k++)
+		if(b[k] >= 0)
 		{
+			const int pos = s_cnt[warp][b[k]] + rank[k];
 			if(pos < ntiles)
-				T.order[pos] = i;
+				T.order[pos] = first + k * 32 + lane;
 			else
 				set_status(a.status, ST_RANGE);
-			if((peers & lanemask_lt()) == 0)
-				cur[b] += __popc(peers);
 		}
-		__syncwarp();
-	}
 }
 
 // Tile of a record given in the FP64 spill layout.
