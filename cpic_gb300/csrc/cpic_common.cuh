@@ -341,6 +341,48 @@ warp_reserve(int32_t *cnt, bool move, int dest)
 	return warp_reserve_finish(warp_reserve_issue(cnt, move, dest), move);
 }
 
+// ------------------------------------- dependent launches in one stream
+//
+// The kernels of a step depend on each other in a chain.  They are launched
+// with programmatic stream serialisation (launch_pdl): a kernel's blocks may
+// start while its predecessor drains, run what touches no data of the
+// chain (shared-memory set-up, constant tables), and wait for the
+// predecessor's completion and memory in pdl_wait().  Every thread of such a
+// kernel calls pdl_wait() before its first access to such data, so a
+// kernel's completion implies that of all before it.  Measured on empty
+// kernels: 1.4 us per dependent launch instead of 3.1.
+__device__ __forceinline__ void pdl_wait()
+{
+	asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Lets the next kernel's blocks start once every block of this one has got
+// here.
+__device__ __forceinline__ void pdl_trigger()
+{
+	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <class T> struct same_type { typedef T type; };
+
+template <typename... A>
+inline cudaError_t launch_pdl(void (*k)(A...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+		typename same_type<A>::type... args)
+{
+	cudaLaunchConfig_t c = {};
+	cudaLaunchAttribute at[1];
+	at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	at[0].val.programmaticStreamSerializationAllowed = 1;
+	c.gridDim = grid;
+	c.blockDim = block;
+	c.dynamicSmemBytes = smem;
+	c.stream = s;
+	c.attrs = at;
+	c.numAttrs = 1;
+	void *argv[] = {(void *) &args...};
+	return cudaLaunchKernelExC(&c, (const void *) k, argv);
+}
+
 // ------------------------------------------------ bulk copies (TMA engine)
 //
 // One thread streams a chunk of each structure-of-arrays column from global
@@ -505,7 +547,19 @@ namespace cpic {
 cudaError_t launch_push_f64(const PushArgs &a, int ntiles, size_t smem, int ppt, cudaStream_t s);
 int push_f64_blocks_per_sm(size_t smem, int ppt);
 void launch_spill_f64(const SpillArgs &a, cudaStream_t s);
-void launch_E_f64(const Grid &g, const double *phi, double *Ex, double *Ey, cudaStream_t s);
+// What the field stage's last kernel clears for the next particle stage:
+// the charge accumulators that stage will add to and its spill-list counts.
+struct NextStage {
+	long long *rho, *rho_lo;     // ny x nx each (rho_lo: FP64 form)
+	int32_t *counts;             // kMaxSpecies of them
+};
+__device__ __forceinline__ void clear_counts(const NextStage &nx)
+{
+	if(blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < kMaxSpecies)
+		nx.counts[threadIdx.x] = 0;
+}
+void launch_E_f64(const Grid &g, const double *phi, double *Ex, double *Ey, const NextStage &nx,
+		cudaStream_t s);
 cudaError_t launch_poisson_f64(const Grid &g, const long long *rho, double qinv,
 		double2 *spec, const double2 *twx, const double2 *twy, double *phi, cudaStream_t s,
 		const long long *rho_lo, double qinv_lo, const double *Gt);
@@ -515,7 +569,7 @@ cudaError_t launch_push_mix(const PushArgs &a, int ntiles, size_t smem, int ppt,
 // memory, for a store with or without ids (0 on error)
 int push_mix_blocks_per_sm(size_t smem, bool ids, int ppt, bool gp2);
 void launch_spill_mix(const SpillArgs &a, cudaStream_t s);
-void launch_E_mix(const Grid &g, const float *phi, float2 *E, cudaStream_t s);
+void launch_E_mix(const Grid &g, const float *phi, float2 *E, const NextStage &nx, cudaStream_t s);
 cudaError_t launch_poisson_mix(const Grid &g, const long long *rho, double qinv, const long long *rsum,
 		float2 *spec, const float2 *twx, const float2 *twy, float *phi, cudaStream_t s, const float *Gt,
 		double mean0 = 0.0);

@@ -71,8 +71,15 @@ struct cpic_ctx {
 	// spill_cur, and writes the other ones
 	int spill_cur;
 	// fields
-	long long *rho;           // ny x nx fixed point
-	long long *rho_lo;        // FP64 form: remainder word (else null)
+	// ny x nx fixed point, and the remainder word (FP64 form, else null):
+	// the current charge, in buffer rho_cur of two.  The field stage clears
+	// the other buffer and the spill counts that the next particle stage
+	// writes (next_clean), which then adds to it and makes it the current one.
+	long long *rho, *rho_lo;
+	long long *rho_buf[2], *rho_lo_buf[2];
+	int rho_cur;
+	bool next_clean;
+	bool spill_empty;         // the spill lists the next stage reads are known to be empty
 	double *phi64, *Ex64, *Ey64;
 	float *phi32;
 	float2 *E32;
@@ -84,15 +91,25 @@ struct cpic_ctx {
 	double *green64;          // Green's function, column order (FP64 form)
 	float *green32;           // same, FP32 (mixed form)
 	double *mean;             // device scalar (mixed form)
+	// one device array: the status word, then the counts of the species'
+	// spill lists 0 and 1 (spill_count), read back in one copy
+	int32_t *ctl;
 	uint32_t *status;
 	double *scratch;          // FP64 scratch for host views / partial sums
 	size_t scratch_n;
 	int32_t *counter;         // device scalar
-	int32_t *probe_h;         // pinned: status word and each species' spill count
+	int32_t *probe_h;         // pinned copy of ctl
+	double *part_h;           // pinned: partial sums of the field energy (2 ny)
 	CUtensorMap emap;         // mixed form: E32 as 2D tiles for the fused kernel
 	bool emap_ok;
 	unsigned long long *counter_pair;  // two device scalars (upload check)
 };
+
+constexpr int kCtl = 1 + 2 * kMaxSpecies;
+static int32_t *spill_count(const cpic_ctx *c, int list, int s)
+{
+	return c->ctl + 1 + list * kMaxSpecies + s;
+}
 
 // ------------------------------------------------------------- kernels
 
@@ -175,6 +192,8 @@ __global__ void __launch_bounds__(kOrderThreads) k_tile_order(const PushArgs a, 
 	__shared__ int32_t s_wsum[kWarps];
 	__shared__ long long s_part[kWarps];
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	pdl_trigger();
+	pdl_wait();
 	// warp w takes tiles [w per, (w + 1) per), 32 at a time
 	const int per = (ntiles + kOrderThreads - 1) / kOrderThreads * 32;
 	const int first = warp * per;
@@ -979,24 +998,27 @@ static void free_store(cpic_ctx *c, SpeciesHost &S, bool alt)
 // The count is cleared on the caller's stream, ahead of the work it
 // queues there (the context's streams do not synchronise with the legacy
 // default stream).
-static int alloc_spill(Spill &S, int32_t capacity, cudaStream_t st, int cell_units = 0)
+// count: the list's counter, null for one of its own.
+static int alloc_spill(Spill &S, int32_t capacity, cudaStream_t st, int cell_units = 0,
+		int32_t *count = nullptr)
 {
 	S.capacity = capacity;
 	S.cell_units = cell_units;
+	S.count = count;
 	CK(cudaMalloc(&S.x, (size_t) capacity * sizeof(double)));
 	CK(cudaMalloc(&S.y, (size_t) capacity * sizeof(double)));
 	CK(cudaMalloc(&S.ux, (size_t) capacity * sizeof(double)));
 	CK(cudaMalloc(&S.uy, (size_t) capacity * sizeof(double)));
 	CK(cudaMalloc(&S.id, (size_t) capacity * sizeof(int32_t)));
-	CK(cudaMalloc(&S.count, sizeof(int32_t)));
+	if(!count) CK(cudaMalloc(&S.count, sizeof(int32_t)));
 	CK(cudaMemsetAsync(S.count, 0, sizeof(int32_t), st));
 	return CPIC_OK;
 }
 
-static void free_spill(Spill &S)
+static void free_spill(Spill &S, bool own_count = true)
 {
 	cudaFree(S.x); cudaFree(S.y); cudaFree(S.ux); cudaFree(S.uy); cudaFree(S.id);
-	cudaFree(S.count);
+	if(own_count) cudaFree(S.count);
 	memset(&S, 0, sizeof(S));
 }
 
@@ -1310,11 +1332,9 @@ static int rebuild_if_spilled(cpic_ctx *c, bool all = true, bool *rebuilt = null
 static int step_check(cpic_ctx *c)
 {
 	cudaStream_t st = c->stream;
-	CK(cudaMemcpyAsync(&c->probe_h[0], c->status, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-	for(int s = 0; s < c->nspecies; s++)
-		CK(cudaMemcpyAsync(&c->probe_h[1 + s], c->sp[s].spill[c->spill_cur].count,
-				sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+	CK(cudaMemcpyAsync(c->probe_h, c->ctl, kCtl * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
 	CK(cudaStreamSynchronize(st));
+	const int32_t *counts = c->probe_h + (spill_count(c, c->spill_cur, 0) - c->ctl);
 	const uint32_t sw = (uint32_t) c->probe_h[0];
 	if(sw & ST_SPILL_FULL) return CPIC_ECAPACITY;
 	if(sw & ST_UMAX) return CPIC_EUMAX;
@@ -1325,9 +1345,10 @@ static int step_check(cpic_ctx *c)
 	c->last_spill = 0;
 	for(int s = 0; s < c->nspecies; s++)
 	{
-		c->last_spill += c->probe_h[1 + s];
-		over = over || c->probe_h[1 + s] > spill_threshold(c, s);
+		c->last_spill += counts[s];
+		over = over || counts[s] > spill_threshold(c, s);
 	}
+	c->spill_empty = c->last_spill == 0;
 	return over ? rebuild_if_spilled(c, false) : CPIC_OK;
 }
 
@@ -1355,12 +1376,19 @@ static int plasma_stage_async(cpic_ctx *c, bool deposit_only, cudaEvent_t ev0 = 
 {
 	cudaStream_t st = c->stream;
 	int64_t ng = (int64_t) c->g.nx * c->g.ny;
-	CK(cudaMemsetAsync(c->rho, 0, ng * sizeof(long long), st));
-	if(c->rho_lo)
-		CK(cudaMemsetAsync(c->rho_lo, 0, ng * sizeof(long long), st));
 	int cur = c->spill_cur;
-	for(int s = 0; s < c->nspecies; s++)
-		CK(cudaMemsetAsync(c->sp[s].spill[cur ^ 1].count, 0, sizeof(int32_t), st));
+	c->rho_cur ^= 1;
+	c->rho = c->rho_buf[c->rho_cur];
+	c->rho_lo = c->rho_lo_buf[c->rho_cur];
+	if(!c->next_clean)
+	{
+		// no field stage since the last particle stage
+		CK(cudaMemsetAsync(c->rho, 0, ng * sizeof(long long), st));
+		if(c->rho_lo)
+			CK(cudaMemsetAsync(c->rho_lo, 0, ng * sizeof(long long), st));
+		CK(cudaMemsetAsync(spill_count(c, cur ^ 1, 0), 0, kMaxSpecies * sizeof(int32_t), st));
+	}
+	c->next_clean = false;
 	SpillArgs sa;
 	memset(&sa, 0, sizeof(sa));
 	sa.p = make_args(c, cur);
@@ -1383,10 +1411,14 @@ static int plasma_stage_async(cpic_ctx *c, bool deposit_only, cudaEvent_t ev0 = 
 	// the spill pass first: its records go to their tiles or to the empty
 	// output list (same capacity as its input), so none can be lost; the
 	// fused kernel's own overflow then falls back to staying in its tile
-	if(c->precision == CPIC_MIXED)
+	// (no pass at all over lists the host has just read as empty)
+	if(c->spill_empty)
+		;
+	else if(c->precision == CPIC_MIXED)
 		launch_spill_mix(sa, st);
 	else
 		launch_spill_f64(sa, st);
+	c->spill_empty = false;
 	if(ev0) CK(cudaEventRecord(ev0, st));
 	if(c->precision == CPIC_MIXED)
 		CK(launch_push_mix(sa.p, c->ntiles, smem, c->ppt, st));
@@ -1399,7 +1431,7 @@ static int plasma_stage_async(cpic_ctx *c, bool deposit_only, cudaEvent_t ev0 = 
 	if(c->order_mode == 0)
 		c->order_mode = tile_order_pays(c, smem) ? 1 : 2;
 	if(c->order_mode == 1)
-		k_tile_order<<<c->nspecies, kOrderThreads, 0, st>>>(sa.p, c->ntiles, cur ^ 1);
+		launch_pdl(k_tile_order, c->nspecies, kOrderThreads, 0, st, sa.p, c->ntiles, cur ^ 1);
 	CK(cudaGetLastError());
 	c->spill_cur ^= 1;
 	return CPIC_OK;
@@ -1430,6 +1462,9 @@ static int normalize(cpic_ctx *c)
 static int field_stage_async(cpic_ctx *c)
 {
 	cudaStream_t st = c->stream;
+	// what the next particle stage adds to, cleared by the last kernel here
+	const NextStage nx = {c->rho_buf[c->rho_cur ^ 1], c->rho_lo_buf[c->rho_cur ^ 1],
+		spill_count(c, c->spill_cur ^ 1, 0)};
 	if(c->precision == CPIC_MIXED)
 	{
 		// the mean charge density the particles carry (each deposits
@@ -1441,15 +1476,16 @@ static int field_stage_async(cpic_ctx *c)
 		double mean0 = tot / ((double) c->g.nx * (double) c->g.ny);
 		CK(launch_poisson_mix(c->g, c->rho, c->qinv, nullptr, c->spec32, c->twx32, c->twy32,
 				c->phi32, st, c->green32, mean0));
-		launch_E_mix(c->g, c->phi32, c->E32, st);
+		launch_E_mix(c->g, c->phi32, c->E32, nx, st);
 	}
 	else
 	{
 		CK(launch_poisson_f64(c->g, c->rho, c->qinv, c->spec64, c->twx64, c->twy64,
 				c->phi64, st, c->rho_lo, c->qinv_lo, c->green64));
-		launch_E_f64(c->g, c->phi64, c->Ex64, c->Ey64, st);
+		launch_E_f64(c->g, c->phi64, c->Ex64, c->Ey64, nx, st);
 	}
 	CK(cudaGetLastError());
+	c->next_clean = true;
 	return CPIC_OK;
 }
 
@@ -1543,18 +1579,22 @@ CPIC_API int cpic_create(const cpic_params_t *p, cpic_ctx_t **out)
 		delete c;
 		return CPIC_ECUDA;
 	}
-	if(cudaMallocHost((void **) &c->probe_h, (1 + kMaxSpecies) * sizeof(int32_t)) != cudaSuccess)
+	// pinned: 2 ny doubles, then the copy of ctl
+	if(cudaMallocHost((void **) &c->part_h, 2 * (size_t) g.ny * sizeof(double) + kCtl * sizeof(int32_t))
+			!= cudaSuccess)
 	{
 		cudaStreamDestroy(c->stream);
 		delete c;
 		return CPIC_ENOMEM;
 	}
+	c->probe_h = reinterpret_cast<int32_t *>(c->part_h + 2 * (size_t) g.ny);
 	int64_t ng = (int64_t) g.nx * g.ny;
 	int64_t nh = g.nx / 2 + 1;
 	int r = CPIC_OK;
 #define AL(ptr, bytes) do { if(cudaMalloc(&(ptr), (bytes)) != cudaSuccess) { r = CPIC_ENOMEM; goto fail; } } while(0)
-	AL(c->rho, ng * sizeof(long long));
-	AL(c->status, sizeof(uint32_t));
+	for(int k = 0; k < 2; k++) AL(c->rho_buf[k], ng * sizeof(long long));
+	AL(c->ctl, kCtl * sizeof(int32_t));
+	c->status = reinterpret_cast<uint32_t *>(c->ctl);
 	AL(c->cosx, g.nx * sizeof(double));
 	AL(c->cosy, g.ny * sizeof(double));
 	AL(c->mean, sizeof(double));
@@ -1563,7 +1603,7 @@ CPIC_API int cpic_create(const cpic_params_t *p, cpic_ctx_t **out)
 	if(c->precision == CPIC_FP64)
 	{
 		AL(c->phi64, ng * sizeof(double));
-		AL(c->rho_lo, ng * sizeof(long long));
+		for(int k = 0; k < 2; k++) AL(c->rho_lo_buf[k], ng * sizeof(long long));
 		AL(c->Ex64, (ng + 3 * (int64_t) g.nx) * sizeof(double));
 		AL(c->Ey64, (ng + 3 * (int64_t) g.nx) * sizeof(double));
 		AL(c->spec64, ng / g.nx * nh * sizeof(double2));
@@ -1583,9 +1623,11 @@ CPIC_API int cpic_create(const cpic_params_t *p, cpic_ctx_t **out)
 		c->emap_ok = encode_field_map(c);
 	}
 #undef AL
+	c->rho = c->rho_buf[0];
+	c->rho_lo = c->rho_lo_buf[0];
 	cudaMemset(c->rho, 0, ng * sizeof(long long));
 	if(c->rho_lo) cudaMemset(c->rho_lo, 0, ng * sizeof(long long));
-	cudaMemset(c->status, 0, sizeof(uint32_t));
+	cudaMemset(c->ctl, 0, kCtl * sizeof(int32_t));
 	{
 		// Green's function cosines as MFT_init computes them
 		// (solver.c:257-278) and FFT twiddles exp(-2 pi i k / n), k < n
@@ -1654,16 +1696,17 @@ CPIC_API void cpic_destroy(cpic_ctx_t *c)
 		cudaFree(S.tiles.base); cudaFree(S.tiles.cap); cudaFree(S.tiles.cnt);
 		cudaFree(S.tiles.abase); cudaFree(S.tiles.acap);
 		cudaFree(S.tiles.acnt[0]); cudaFree(S.tiles.acnt[1]); cudaFree(S.tiles.order);
-		free_spill(S.spill[0]);
-		free_spill(S.spill[1]);
+		free_spill(S.spill[0], false);
+		free_spill(S.spill[1], false);
 	}
-	cudaFree(c->rho); cudaFree(c->rho_lo); cudaFree(c->phi64); cudaFree(c->Ex64); cudaFree(c->Ey64);
+	for(int k = 0; k < 2; k++) { cudaFree(c->rho_buf[k]); cudaFree(c->rho_lo_buf[k]); }
+	cudaFree(c->phi64); cudaFree(c->Ex64); cudaFree(c->Ey64);
 	cudaFree(c->phi32); cudaFree(c->E32); cudaFree(c->spec64); cudaFree(c->spec32);
 	cudaFree(c->twx64); cudaFree(c->twy64); cudaFree(c->twx32); cudaFree(c->twy32);
 	cudaFree(c->cosx); cudaFree(c->cosy); cudaFree(c->green64); cudaFree(c->green32); cudaFree(c->mean);
-	cudaFree(c->status); cudaFree(c->scratch); cudaFree(c->counter); cudaFree(c->counter_pair);
+	cudaFree(c->ctl); cudaFree(c->scratch); cudaFree(c->counter); cudaFree(c->counter_pair);
 	if(c->stream) cudaStreamDestroy(c->stream);
-	if(c->probe_h) cudaFreeHost(c->probe_h);
+	if(c->part_h) cudaFreeHost(c->part_h);
 	delete c;
 }
 
@@ -1799,8 +1842,8 @@ CPIC_API int cpic_add_species(cpic_ctx_t *c, double q, double m, int64_t n,
 	// room for an eighth of the species to overflow between two host checks
 	int32_t scap = (int32_t) std::max<int64_t>(65536, n / 8);
 	const int cu = c->precision == CPIC_MIXED ? 1 : 0;
-	if((r = alloc_spill(S.spill[0], scap, st, cu))) return r;
-	if((r = alloc_spill(S.spill[1], scap, st, cu))) return r;
+	if((r = alloc_spill(S.spill[0], scap, st, cu, spill_count(c, 0, s)))) return r;
+	if((r = alloc_spill(S.spill[1], scap, st, cu, spill_count(c, 1, s)))) return r;
 	c->nspecies++;
 
 	// counting sort of the staged particles into the tiles
@@ -2146,10 +2189,10 @@ CPIC_API int cpic_field_energy(cpic_ctx_t *c, double *out)
 	int r = ensure_scratch(c, 2 * (size_t) ny);
 	if(r) return r;
 	cudaStream_t st = c->stream;
-	std::vector<double> h(2 * (size_t) ny);
+	const double *h = c->part_h;
 	k_field_energy<<<ny, 256, 0, st>>>(c->g, c->Ex64, c->Ey64,
 			c->precision == CPIC_MIXED ? c->E32 : nullptr, c->rho, c->scratch);
-	CK(cudaMemcpyAsync(h.data(), c->scratch, 2 * ny * sizeof(double), cudaMemcpyDeviceToHost, st));
+	CK(cudaMemcpyAsync(c->part_h, c->scratch, 2 * ny * sizeof(double), cudaMemcpyDeviceToHost, st));
 	CK(cudaStreamSynchronize(st));
 	double we = 0.0, q = 0.0;
 	for(int i = 0; i < ny; i++) { we += h[2 * i]; q += h[2 * i + 1]; }
@@ -2359,6 +2402,7 @@ static std::vector<const void *> ens_sig(const cpic_ensemble *e)
 	for(const cpic_ctx *c : e->runs)
 	{
 		v.push_back(reinterpret_cast<const void *>((uintptr_t) c->spill_cur));
+		v.push_back(c->rho);
 		for(int s = 0; s < c->nspecies; s++)
 		{
 			v.push_back(c->sp[s].f64.x);
@@ -2388,6 +2432,7 @@ static int ens_capture(cpic_ensemble *e)
 	{
 		cpic_ctx *c = e->runs[i];
 		if(cudaStreamWaitEvent(c->stream, e->fork, 0) != cudaSuccess) { r = CPIC_ECUDA; break; }
+		c->spill_empty = false;          // the graph runs for any spill lists
 		for(int k = 0; k < 2 && r == CPIC_OK; k++)
 		{
 			r = field_stage_async(c);

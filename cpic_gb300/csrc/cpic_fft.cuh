@@ -554,7 +554,9 @@ static __global__ void k_rows_fwd(const __grid_constant__ FftPlan px, int ny, co
 	const int nx = px.n;
 	C *a = reinterpret_cast<C *>(smem_raw);
 	C *b = a + nx;
+	pdl_trigger();
 	tw = fft_tw_stage(b + nx, tw, fft_tw_elems(px), tw_sm);
+	pdl_wait();
 	int r0 = 2 * blockIdx.x;
 	const bool two = r0 + 1 < ny;            // an odd ny leaves the last row alone
 	int nh = nx / 2 + 1;
@@ -615,7 +617,9 @@ __device__ __forceinline__ void cols_body(const FftPlan &py, int nh, int cb, typ
 	const int pitch = fft_pitch(ny, cb);
 	C *a = reinterpret_cast<C *>(smem_raw);
 	C *b = a + (size_t) cb * pitch;
+	pdl_trigger();
 	tw = fft_tw_stage(b + (size_t) cb * pitch, tw, fft_tw_elems(py), tw_sm, twsh);
+	pdl_wait();
 	// element idx of the block's columns: row idx / ncol, column idx % ncol
 	// (cb is 1, 2 or 4; a last block with fewer columns divides)
 	const int lg = (ncol & (ncol - 1)) == 0 ? __ffs(ncol) - 1 : -1;
@@ -668,7 +672,9 @@ static __global__ void k_rows_inv(const __grid_constant__ FftPlan px, int ny,
 	const int nx = px.n;
 	C *a = reinterpret_cast<C *>(smem_raw);
 	C *b = a + nx;
+	pdl_trigger();
 	tw = fft_tw_stage(b + nx, tw, fft_tw_elems(px), tw_sm, twsh);
+	pdl_wait();
 	int r0 = 2 * blockIdx.x;
 	const bool two = r0 + 1 < ny;            // an odd ny leaves the last row alone
 	int nh = nx / 2 + 1;
@@ -715,7 +721,9 @@ static __global__ void k_rows_fwd_real(const __grid_constant__ FftPlan px, int n
 	const int nx = px.n;
 	C *a = reinterpret_cast<C *>(smem_raw);
 	C *b = a + nx;
+	pdl_trigger();
 	tw = fft_tw_stage(b + nx, tw, fft_tw_elems(px), tw_sm, twsh);
+	pdl_wait();
 	int r0 = 2 * blockIdx.x;
 	const bool two = r0 + 1 < ny;
 	int nh = nx / 2 + 1;
@@ -782,9 +790,9 @@ static void poisson_tail(int nx, int ny, const FftPlan &px, const FftPlan &py, c
 {
 	const int nh = nx / 2 + 1;
 	const FftShape cs = fft_shape<T>(py, cols_per_block<T>(nh, ny));
-	k_cols<T><<<(nh + cs.nb - 1) / cs.nb, cs.threads, cs.smem, s>>>(py, nh, cs.nb, spec, twy, Gt,
+	launch_pdl(k_cols<T>, (nh + cs.nb - 1) / cs.nb, cs.threads, cs.smem, s, py, nh, cs.nb, spec, twy, Gt,
 			cs.tw_sm);
-	k_rows_inv<T><<<(ny + 1) / 2, rs.threads, rs.smem, s>>>(px, ny, spec, twx, phi, rs.tw_sm,
+	launch_pdl(k_rows_inv<T>, (ny + 1) / 2, rs.threads, rs.smem, s, px, ny, spec, twx, phi, rs.tw_sm,
 			node_count<T>(nx, ny), 0);
 }
 
@@ -797,7 +805,7 @@ static void poisson_launch(const Grid &g, const long long *rho, double qinv, con
 {
 	const FftPlan px = fft_plan(g.nx), py = fft_plan(g.ny);
 	const FftShape rs = fft_shape<T>(px, 1);
-	k_rows_fwd<T><<<(g.ny + 1) / 2, rs.threads, rs.smem, s>>>(px, g.ny, rho, qinv, mean, spec, twx,
+	launch_pdl(k_rows_fwd<T>, (g.ny + 1) / 2, rs.threads, rs.smem, s, px, g.ny, rho, qinv, mean, spec, twx,
 			rho_lo, qinv_lo, mean0, rs.tw_sm, node_count<double>(g.nx, g.ny));
 	poisson_tail<T>(g.nx, g.ny, px, py, rs, spec, twx, twy, Gt, phi, s);
 }
@@ -811,7 +819,8 @@ static void poisson_launch_real(int nx, int ny, const T *in, typename Cx<T>::t *
 {
 	const FftPlan px = fft_plan(nx), py = fft_plan(ny);
 	const FftShape rs = fft_shape<T>(px, 1);
-	k_rows_fwd_real<T><<<(ny + 1) / 2, rs.threads, rs.smem, s>>>(px, ny, in, spec, twx, rs.tw_sm, 0);
+	launch_pdl(k_rows_fwd_real<T>, (ny + 1) / 2, rs.threads, rs.smem, s, px, ny, in, spec, twx, rs.tw_sm,
+			0);
 	poisson_tail<T>(nx, ny, px, py, rs, spec, twx, twy, Gt, out, s);
 }
 

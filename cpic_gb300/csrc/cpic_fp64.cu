@@ -14,8 +14,12 @@ namespace cpic {
 // The divisions by 2 dx and 2 dy are bits::div_by (the quotient's value, three
 // FP64 instructions each: two divisions per node took 9 of the kernel's 12
 // us on a 512 x 512 grid).
-__global__ void k_E_f64(Grid g, const double *phi, double *Ex, double *Ey, double rdx2, double rdy2)
+__global__ void k_E_f64(Grid g, const double *phi, double *Ex, double *Ey, double rdx2, double rdy2,
+		const NextStage next)
 {
+	pdl_trigger();
+	pdl_wait();
+	clear_counts(next);
 	double dx2 = 2 * g.dx, dy2 = 2 * g.dy;
 	// rows 0..ny over blockIdx.y (row ny is the south ghost: row 0 again)
 	for(int iy = blockIdx.y; iy <= g.ny; iy += gridDim.y)
@@ -29,17 +33,23 @@ __global__ void k_E_f64(Grid g, const double *phi, double *Ex, double *Ey, doubl
 			int x0 = ix == 0 ? g.nx - 1 : ix - 1;
 			int x1 = ix + 1 == g.nx ? 0 : ix + 1;
 			int64_t i = (int64_t) iy * g.nx + ix;
+			if(iy < g.ny)
+			{
+				next.rho[i] = 0;
+				next.rho_lo[i] = 0;
+			}
 			Ey[i] = bits::div_by(phi[(int64_t) y0 * g.nx + ix] - phi[(int64_t) y1 * g.nx + ix], dy2, rdy2);
 			Ex[i] = bits::div_by(phi[(int64_t) yc * g.nx + x0] - phi[(int64_t) yc * g.nx + x1], dx2, rdx2);
 		}
 	}
 }
 
-void launch_E_f64(const Grid &g, const double *phi, double *Ex, double *Ey, cudaStream_t s)
+void launch_E_f64(const Grid &g, const double *phi, double *Ex, double *Ey, const NextStage &nx,
+		cudaStream_t s)
 {
 	dim3 grid((g.nx + 255) / 256, 1);
 	grid.y = (unsigned) std::min(g.ny + 1, std::max(1, 4096 / (int) grid.x));
-	k_E_f64<<<grid, 256, 0, s>>>(g, phi, Ex, Ey, 1.0 / (2 * g.dx), 1.0 / (2 * g.dy));
+	launch_pdl(k_E_f64, grid, 256, 0, s, g, phi, Ex, Ey, 1.0 / (2 * g.dx), 1.0 / (2 * g.dy), nx);
 }
 
 // E at every particle (interpolate_f2p_E), written by particle id.  One
@@ -112,16 +122,16 @@ cudaError_t launch_push_f64(const PushArgs &a, int ntiles, size_t smem, int ppt,
 	for(int sp = 0; sp < a.nspecies; sp++)
 	{
 		const PushArgs b = species_args(a, sp);
-		if(ppt == 1) k_push<F64, F64::min_blocks(1), true, 1><<<ntiles, kPushThreads, smem, s>>>(b);
-		else if(ppt == 4) k_push<F64, F64::min_blocks(4), true, 4><<<ntiles, kPushThreads, smem, s>>>(b);
-		else k_push<F64, F64::min_blocks(2), true, 2><<<ntiles, kPushThreads, smem, s>>>(b);
+		if(ppt == 1) launch_pdl(k_push<F64, F64::min_blocks(1), true, 1>, ntiles, kPushThreads, smem, s, b);
+		else if(ppt == 4) launch_pdl(k_push<F64, F64::min_blocks(4), true, 4>, ntiles, kPushThreads, smem, s, b);
+		else launch_pdl(k_push<F64, F64::min_blocks(2), true, 2>, ntiles, kPushThreads, smem, s, b);
 	}
 	return cudaSuccess;
 }
 
 void launch_spill_f64(const SpillArgs &a, cudaStream_t s)
 {
-	k_spill<F64><<<152, kPushThreads, 0, s>>>(a);
+	launch_pdl(k_spill<F64>, 152, kPushThreads, 0, s, a);
 }
 
 cudaError_t launch_poisson_f64(const Grid &g, const long long *rho, double qinv,

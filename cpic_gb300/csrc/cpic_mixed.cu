@@ -11,8 +11,11 @@ namespace cpic {
 // E = -grad(phi), FP32, periodic (field_E_compute, src/field.c:358-416),
 // stored as (Ex, Ey) pairs for the per-tile shared-memory stage.  Rows
 // over blockIdx.y, so no index is divided.
-__global__ void k_E_mix(Grid g, const float *phi, float2 *E)
+__global__ void k_E_mix(Grid g, const float *phi, float2 *E, const NextStage next)
 {
+	pdl_trigger();
+	pdl_wait();
+	clear_counts(next);
 	// four nodes of one row per thread (nx a multiple of 4): one float4 of
 	// phi from each of the three rows, the two x neighbours outside it,
 	// two float4 stores of E
@@ -40,13 +43,19 @@ __global__ void k_E_mix(Grid g, const float *phi, float2 *E)
 			float4 *o = reinterpret_cast<float4 *>(E + (int64_t) iy * g.nx + x);
 			o[0] = e0;
 			o[1] = e1;
+			longlong2 *z = reinterpret_cast<longlong2 *>(next.rho + (int64_t) iy * g.nx + x);
+			z[0] = make_longlong2(0, 0);
+			z[1] = make_longlong2(0, 0);
 		}
 	}
 }
 
 // The same for any nx: one node per thread.
-__global__ void k_E_mix_any(Grid g, const float *phi, float2 *E)
+__global__ void k_E_mix_any(Grid g, const float *phi, float2 *E, const NextStage next)
 {
+	pdl_trigger();
+	pdl_wait();
+	clear_counts(next);
 	const float rdx2 = (float) (1.0 / (2 * g.dx)), rdy2 = (float) (1.0 / (2 * g.dy));
 	for(int iy = blockIdx.y; iy < g.ny; iy += gridDim.y)
 	{
@@ -60,18 +69,18 @@ __global__ void k_E_mix_any(Grid g, const float *phi, float2 *E)
 			e.x = (r[xm] - r[xp]) * rdx2;
 			e.y = (phi[(int64_t) y0 * g.nx + x] - phi[(int64_t) y1 * g.nx + x]) * rdy2;
 			E[(int64_t) iy * g.nx + x] = e;
+			next.rho[(int64_t) iy * g.nx + x] = 0;
 		}
 	}
 }
 
-void launch_E_mix(const Grid &g, const float *phi, float2 *E, cudaStream_t s)
+void launch_E_mix(const Grid &g, const float *phi, float2 *E, const NextStage &nx, cudaStream_t s)
 {
 	const bool quads = g.nx % 4 == 0;
 	const int per_row = quads ? g.nx >> 2 : g.nx;
 	dim3 grid((per_row + 255) / 256, 1);
 	grid.y = (unsigned) std::min(g.ny, std::max(1, 8 * 152 / (int) grid.x));
-	if(quads) k_E_mix<<<grid, 256, 0, s>>>(g, phi, E);
-	else k_E_mix_any<<<grid, 256, 0, s>>>(g, phi, E);
+	launch_pdl(quads ? k_E_mix : k_E_mix_any, grid, 256, 0, s, g, phi, E, nx);
 }
 
 // E at every particle of a mixed store, by particle id (ids required).
@@ -180,13 +189,13 @@ static void launch_push_mix_pg(const PushArgs &b, int ntiles, size_t smem, bool 
 {
 	if(ids)
 	{
-		if(hi) k_push<Mix, Mix::kHiBlocks, true, P, G><<<ntiles, kPushThreads, smem, s>>>(b);
-		else k_push<Mix, Mix::kMinBlocks, true, P, G><<<ntiles, kPushThreads, smem, s>>>(b);
+		if(hi) launch_pdl(k_push<Mix, Mix::kHiBlocks, true, P, G>, ntiles, kPushThreads, smem, s, b);
+		else launch_pdl(k_push<Mix, Mix::kMinBlocks, true, P, G>, ntiles, kPushThreads, smem, s, b);
 	}
 	else
 	{
-		if(hi) k_push<Mix, Mix::kHiBlocks, false, P, G><<<ntiles, kPushThreads, smem, s>>>(b);
-		else k_push<Mix, Mix::kMinBlocks, false, P, G><<<ntiles, kPushThreads, smem, s>>>(b);
+		if(hi) launch_pdl(k_push<Mix, Mix::kHiBlocks, false, P, G>, ntiles, kPushThreads, smem, s, b);
+		else launch_pdl(k_push<Mix, Mix::kMinBlocks, false, P, G>, ntiles, kPushThreads, smem, s, b);
 	}
 }
 
@@ -217,7 +226,7 @@ cudaError_t launch_push_mix(const PushArgs &a, int ntiles, size_t smem, int ppt,
 
 void launch_spill_mix(const SpillArgs &a, cudaStream_t s)
 {
-	k_spill<Mix><<<152, kPushThreads, 0, s>>>(a);
+	launch_pdl(k_spill<Mix>, 152, kPushThreads, 0, s, a);
 }
 
 cudaError_t launch_poisson_mix(const Grid &g, const long long *rho, double qinv, const long long *mean,

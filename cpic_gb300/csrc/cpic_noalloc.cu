@@ -135,18 +135,6 @@ static int scratch_for_current_device(void **out, cudaStream_t s)
 	return CPIC_OK;
 }
 
-// One launch with its own error code (cudaLaunchKernel reports this launch's
-// configuration error, not an earlier one left pending on the thread).
-template <class T> struct same { typedef T type; };
-
-template <typename... A>
-static cudaError_t launch(void (*k)(A...), int blocks, int threads, size_t smem, cudaStream_t s,
-		typename same<A>::type... args)
-{
-	void *argv[] = {(void *) &args...};
-	return cudaLaunchKernel((const void *) k, dim3(blocks), dim3(threads), argv, smem, s);
-}
-
 } // namespace
 
 extern "C" CPIC_API int
@@ -173,13 +161,21 @@ cpic_poisson_noalloc(const double *rho, double *phi, int64_t nx, int64_t ny, voi
 	const int sx = kLog2MaxN - px.log2n;
 
 	// one column per block, at most 257 of them
-	cudaError_t e = launch(k_rows_fwd_real<double>, nyi / 2, rs.threads, rs.smem, s, px, nyi, rho, spec,
-			tw, true, sx);
+	// (each launch reports its own error, not an earlier one left pending on
+	// the thread).  The first one waits for whatever the caller has queued in
+	// the ordinary way: that may be any operation, or the table's launch.
+	double2 *spec0 = spec;
+	bool kept = true;
+	int nyarg = nyi, sharg = sx;
+	FftPlan pxarg = px;
+	void *argv[] = {&pxarg, &nyarg, (void *) &rho, &spec0, (void *) &tw, &kept, &sharg};
+	cudaError_t e = cudaLaunchKernel((const void *) k_rows_fwd_real<double>, dim3(nyi / 2),
+			dim3(rs.threads), argv, rs.smem, s);
 	if(e == cudaSuccess)
-		e = launch(k_noalloc_cols, nh, cs.threads, cs.smem + (nyi / 2 + 1) * sizeof(double), s, py, nh,
+		e = launch_pdl(k_noalloc_cols, nh, cs.threads, cs.smem + (nyi / 2 + 1) * sizeof(double), s, py, nh,
 				px.log2n, spec, tw, cs.smem);
 	if(e == cudaSuccess)
-		e = launch(k_rows_inv<double>, nyi / 2, rs.threads, rs.smem, s, px, nyi, spec, tw, phi, true,
+		e = launch_pdl(k_rows_inv<double>, nyi / 2, rs.threads, rs.smem, s, px, nyi, spec, tw, phi, true,
 				node_count<double>(nxi, nyi), sx);
 	if(e != cudaSuccess)
 	{

@@ -899,20 +899,8 @@ k_push(const __grid_constant__ PushArgs a)
 	// has a fixed offset (no indexed constant loads in the particle loop)
 	const int s = 0;
 	const Tiles &T = a.tiles[s];
-	// blocks are dispatched in index order; the order array puts the
-	// heaviest tiles first (a permutation, so every tile is taken once)
-	const int t = T.order ? T.order[blockIdx.x] : (int) blockIdx.x;
-	if((unsigned) t >= gridDim.x)
-	{
-		if(threadIdx.x == 0) set_status(a.status, ST_RANGE);
-		return;
-	}
 	const int H = g.halo;
 	const int W = g.tx + 2 * H + 1;
-	int ttx, tty;
-	tile_rc(g, t, ttx, tty);
-	const int tx0 = ttx << g.ltx;
-	const int ty0 = tty << g.lty;
 	const bool ids = Ids;
 	const size_t sb = F::stage_bytes(ids, kChunk);
 	// bulk-copy destinations need 16-byte alignment; the host adds 128
@@ -923,7 +911,34 @@ k_push(const __grid_constant__ PushArgs a)
 		+ ((128u - (unsigned) (reinterpret_cast<uintptr_t>(smem) & 127u)) & 127u);
 	unsigned char *fsm = stage0 + 2 * sb;
 
+	// barriers set up while the previous kernel drains
+	pdl_trigger();
+	if(threadIdx.x == 0)
+	{
+		s_cursor = 0;
+		s_timeout = 0;
+		mbar_init(&bars[0], 1);          // "full": one arrival + bytes
+		mbar_init(&bars[1], 1);
+		mbar_init(&ebars[0], kPushThreads / 32);   // "empty": one per warp
+		mbar_init(&ebars[1], kPushThreads / 32);
+		mbar_init(&fbar, 1);
+		fence_mbar_init();
+	}
+	pdl_wait();
+
+	// blocks are dispatched in index order; the order array puts the
+	// heaviest tiles first (a permutation, so every tile is taken once)
+	const int t = T.order ? T.order[blockIdx.x] : (int) blockIdx.x;
 	F::clear(fsm, W, g.tx);
+	if((unsigned) t >= gridDim.x)
+	{
+		if(threadIdx.x == 0) set_status(a.status, ST_RANGE);
+		return;
+	}
+	int ttx, tty;
+	tile_rc(g, t, ttx, tty);
+	const int tx0 = ttx << g.ltx;
+	const int ty0 = tty << g.lty;
 	// the field tile: one 2D tensor copy (issued with the barriers below)
 	// where the form has a map for it, else per-thread loads
 	const bool ftma = F::field_tma(a, tx0, ty0);
@@ -965,19 +980,8 @@ k_push(const __grid_constant__ PushArgs a)
 		s_nbase[threadIdx.x] = T.abase[nt] + aofs_w;
 		s_ncap[threadIdx.x] = T.acap[nt];
 	}
-	if(threadIdx.x == 0)
-	{
-		s_cursor = 0;
-		s_timeout = 0;
-		mbar_init(&bars[0], 1);          // "full": one arrival + bytes
-		mbar_init(&bars[1], 1);
-		mbar_init(&ebars[0], kPushThreads / 32);   // "empty": one per warp
-		mbar_init(&ebars[1], kPushThreads / 32);
-		mbar_init(&fbar, 1);
-		fence_mbar_init();
-		if(ftma)
-			F::field_issue(a, fsm, tx0, ty0, &fbar);
-	}
+	if(threadIdx.x == 0 && ftma)
+		F::field_issue(a, fsm, tx0, ty0, &fbar);
 	__syncthreads();
 	if(threadIdx.x == 0 && nchunks > 0)
 	{
@@ -1178,6 +1182,8 @@ k_spill(const SpillArgs sa)
 {
 	const PushArgs &a = sa.p;
 	const Grid &g = a.g;
+	pdl_trigger();
+	pdl_wait();
 	for(int s = 0; s < a.nspecies; s++)
 	{
 		const Spill &S = sa.spill_in[s];
