@@ -881,6 +881,49 @@ static bool encode_field_map(cpic_ctx *c)
 			CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Tiles of T x T cells.  T need not divide the grid: the tiles of the last
+// column and row are then partly outside it, where no particle lies.
+static void set_tiles(cpic_ctx *c, int T)
+{
+	Grid &g = c->g;
+	g.tx = g.ty = T;
+	g.ntx = (g.nx + T - 1) / T;
+	g.nty = (g.ny + T - 1) / T;
+	g.ltx = g.lty = ilog2(T);
+	bits::div_init((uint32_t) g.ntx, g.ntx_mul, g.ntx_sh);
+	c->ntiles = g.ntx * g.nty;
+	c->emap_ok = c->E32 != nullptr && encode_field_map(c);
+}
+
+// The library's tile size for n particles of one species: the largest of 32,
+// 16, 8 and 4 cells whose tiles keep the SMs busy to the end.  One block takes
+// a tile, an SM holds 5 or 6 of them, and a block alone on an SM works off
+// its particles at a fraction of the SM's rate, so: over two waves of tiles
+// (2048), whatever they hold; about a wave (912) if none takes long (8192
+// particles, FP64 2048: its particles take four times as long); a tile per
+// SM if each is short; or next to nothing per tile, where launch latency is
+// all there is.  Smaller tiles than that only add edges.  Measured (particle
+// kernel, us per step, mixed unless said): 128 x 128 with 128 per cell,
+// 16-cell tiles 113, 8-cell 40, 4-cell 31; 256 x 256 with 32, 16-cell 40,
+// 8-cell 31, 4-cell 38; 512 x 512 with 4, 16-cell 25, 8-cell 31, with 100,
+// 16-cell 241, 8-cell 222; 1024 x 1024 with 25, 32-cell 252, 16-cell 233;
+// 2048 x 2048 with 6, 64-cell 402, 32-cell 254, 16-cell 324; FP64 64 x 64
+// with 64, 8-cell 111, 4-cell 46; FP64 512 x 512 with 16, 16-cell 723,
+// 8-cell 690, 4-cell 824.
+static int auto_tile(const cpic_params_t *p, int64_t n)
+{
+	const bool f64 = p->precision == CPIC_FP64;
+	for(int T = 32; T > 4; T >>= 1)
+	{
+		const int64_t tiles = ((p->nx + T - 1) / T) * ((p->ny + T - 1) / T);
+		const int64_t per = n / tiles;
+		if(tiles >= 2048 || (tiles >= 912 && per <= (f64 ? 2048 : 8192))
+				|| (tiles >= 152 && per <= (f64 ? 512 : 1024)) || per <= 128)
+			return T;
+	}
+	return 4;
+}
+
 static void fill_species_step(cpic_ctx *c, PushArgs &a, int64_t iter)
 {
 	const cpic_params_t &p = c->p;
@@ -1538,24 +1581,10 @@ CPIC_API int cpic_create(const cpic_params_t *p, cpic_ctx_t **out)
 	// interpolate_f2p_E / interpolate_p2f_rho, interpolate.c:303-304
 	g.idx = 1.0 / g.dx;
 	g.idy = 1.0 / g.dy;
-	int T = p->tile_x;
-	if(T <= 0)
-	{
-		// default: the largest tile with at least 2048 tiles, else the
-		// largest tile giving at least 64 tiles, else the largest power of
-		// two up to 32 dividing both sides (1 for an odd side)
-		T = 0;
-		for(int cand = 64; cand >= 4 && !T; cand >>= 1)
-			if(p->nx % cand == 0 && p->ny % cand == 0
-					&& (p->nx / cand) * (p->ny / cand) >= 2048) T = cand;
-		for(int cand = 32; cand >= 4 && !T; cand >>= 1)
-			if(p->nx % cand == 0 && p->ny % cand == 0
-					&& (p->nx / cand) * (p->ny / cand) >= 64) T = cand;
-		for(int cand = 32; cand >= 1 && !T; cand >>= 1)
-			if(p->nx % cand == 0 && p->ny % cand == 0) T = cand;
-	}
+	// (chosen again by the particles of the first species)
+	const int T = p->tile_x > 0 ? p->tile_x : auto_tile(p, 0);
 	int TY = p->tile_y > 0 ? p->tile_y : T;
-	if(!pow2(T) || !pow2(TY) || p->nx % T || p->ny % TY || T != TY)
+	if(!pow2(T) || !pow2(TY) || (p->tile_x > 0 && (p->nx % T || p->ny % TY)) || T != TY)
 	{
 		delete c;
 		return CPIC_EINVAL;
@@ -1566,14 +1595,10 @@ CPIC_API int cpic_create(const cpic_params_t *p, cpic_ctx_t **out)
 		delete c;
 		return CPIC_EINVAL;
 	}
-	g.tx = T; g.ty = TY;
-	g.ntx = g.nx / T; g.nty = g.ny / TY;
 	g.halo = p->halo > 0 ? p->halo : 2;
 	g.lcx = ilog2(g.nx);
-	g.ltx = ilog2(T); g.lty = ilog2(TY);
-	bits::div_init((uint32_t) g.ntx, g.ntx_mul, g.ntx_sh);
 	g.pow2 = pow2(g.nx) && pow2(g.ny);
-	c->ntiles = g.ntx * g.nty;
+	set_tiles(c, T);
 	if(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess)
 	{
 		delete c;
@@ -1620,7 +1645,7 @@ CPIC_API int cpic_create(const cpic_params_t *p, cpic_ctx_t **out)
 		AL(c->twx32, g.nx * sizeof(float2));
 		AL(c->twy32, g.ny * sizeof(float2));
 		cudaMemset(c->E32, 0, ng * sizeof(float2));
-		c->emap_ok = encode_field_map(c);
+		set_tiles(c, T);
 	}
 #undef AL
 	c->rho = c->rho_buf[0];
@@ -1803,6 +1828,8 @@ CPIC_API int cpic_add_species(cpic_ctx_t *c, double q, double m, int64_t n,
 	}
 
 	int s = c->nspecies;
+	if(s == 0 && n > 0 && c->p.tile_x <= 0)
+		set_tiles(c, auto_tile(&c->p, n));
 	SpeciesHost &S = c->sp[s];
 	memset((void *) &S, 0, sizeof(S));
 	S.q = q; S.m = m; S.n = n;
@@ -1813,13 +1840,12 @@ CPIC_API int cpic_add_species(cpic_ctx_t *c, double q, double m, int64_t n,
 	// instruction cache (two-stream 512x512, 100 per cell: 1911 us per launch
 	// with 1, 2503 with 2; two species, 16 per cell: 357 and 470).
 	// Mixed: 1 while every species has fewer than kSmallTile particles per
-	// tile, else 2 (chunks of 512).  A tile's last main-region chunk and its
-	// arrivals chunk are partial, and on small tiles they and the latency
-	// between chunks dominate; two-stream 2048x2048 (102,400 per tile) is
-	// fastest with 2.
+	// tile, else 2 (chunks of 512): 256 x 256 with 512 per tile 17.6 us with
+	// 1, 17.1 with 2, with 2048 per tile 35.0 and 31.0; 128 x 128 with 512
+	// per tile 10.6 and 12.1; 64 x 64 with 128 per tile 8.7 and 10.4.
 	if(c->p.particles_per_thread <= 0)
 	{
-		constexpr int64_t kSmallTile = 4096;
+		constexpr int64_t kSmallTile = 1024;
 		bool small = n / std::max(1, c->ntiles) < kSmallTile;
 		for(int k = 0; k < c->nspecies; k++)
 			small = small && c->sp[k].n / std::max(1, c->ntiles) < kSmallTile;

@@ -31,6 +31,20 @@
 
 namespace cpic {
 
+// Bytes of a bulk copy: a multiple of 16 (reads up to 12 bytes of spare
+// slots past the last particle).
+__device__ __forceinline__ uint32_t round16(int bytes) { return (uint32_t) ((bytes + 15) & ~15); }
+
+// One chunk of a tile's particles in the stage: n from slot `first` of the
+// store at the front, then na from slot `afirst` in the stage's slots from
+// aslot() on (a multiple of 4, so that every column's copy starts on a 16-byte
+// boundary).
+struct Chunk {
+	int64_t first, afirst;
+	int n, na;
+	__device__ __forceinline__ int aslot() const { return (n + 3) & ~3; }
+};
+
 // =================================================================== F64
 
 struct F64 {
@@ -91,20 +105,29 @@ struct F64 {
 		return (size_t) C * (4 * sizeof(double) + sizeof(int32_t));
 	}
 
-	// Thread 0: arm `bar` and copy particles [c0, c0 + cnt) of the tile.
+	// Thread 0: arm `bar` and copy the chunk's particles into the stage.
 	template <int C>
-	static __device__ __forceinline__ void stage_issue(const PushArgs &a, int s, int64_t first,
-			int cnt, unsigned char *buf, uint64_t *bar)
+	static __device__ __forceinline__ void stage_issue(const PushArgs &a, int s, const Chunk &k,
+			unsigned char *buf, uint64_t *bar)
 	{
 		const StoreF64 &st = a.f64[s];
-		uint32_t b8 = (uint32_t) ((cnt * 8 + 15) & ~15);
-		uint32_t b4 = (uint32_t) ((cnt * 4 + 15) & ~15);
-		mbar_arrive_expect_tx(bar, 4 * b8 + b4);
-		bulk_g2s(buf, st.x + first, b8, bar);
-		bulk_g2s(buf + C * 8, st.y + first, b8, bar);
-		bulk_g2s(buf + C * 16, st.ux + first, b8, bar);
-		bulk_g2s(buf + C * 24, st.uy + first, b8, bar);
-		bulk_g2s(buf + C * 32, st.id + first, b4, bar);
+		const uint32_t b8 = round16(k.n * 8), b4 = round16(k.n * 4);
+		const uint32_t a8 = round16(k.na * 8), a4 = round16(k.na * 4);
+		mbar_arrive_expect_tx(bar, 4 * (b8 + a8) + b4 + a4);
+		bulk_g2s(buf, st.x + k.first, b8, bar);
+		bulk_g2s(buf + C * 8, st.y + k.first, b8, bar);
+		bulk_g2s(buf + C * 16, st.ux + k.first, b8, bar);
+		bulk_g2s(buf + C * 24, st.uy + k.first, b8, bar);
+		bulk_g2s(buf + C * 32, st.id + k.first, b4, bar);
+		if(k.na)
+		{
+			buf += 8 * k.aslot();
+			bulk_g2s(buf, st.x + k.afirst, a8, bar);
+			bulk_g2s(buf + C * 8, st.y + k.afirst, a8, bar);
+			bulk_g2s(buf + C * 16, st.ux + k.afirst, a8, bar);
+			bulk_g2s(buf + C * 24, st.uy + k.afirst, a8, bar);
+			bulk_g2s(buf + C * 32 - 4 * k.aslot(), st.id + k.afirst, a4, bar);
+		}
 	}
 
 	template <int C>
@@ -547,17 +570,24 @@ struct Mix {
 	}
 
 	template <int C>
-	static __device__ __forceinline__ void stage_issue(const PushArgs &a, int s, int64_t first,
-			int cnt, unsigned char *buf, uint64_t *bar)
+	static __device__ __forceinline__ void stage_issue(const PushArgs &a, int s, const Chunk &k,
+			unsigned char *buf, uint64_t *bar)
 	{
 		const StoreMix &st = a.mix[s];
-		uint32_t b4 = (uint32_t) ((cnt * 4 + 15) & ~15);
-		uint32_t b16 = (uint32_t) cnt * 16;
-		mbar_arrive_expect_tx(bar, (st.id ? 2 : 1) * b4 + b16);
-		bulk_g2s(buf, st.cell + first, b4, bar);
-		bulk_g2s(buf + C * 4, st.ou + first, b16, bar);
+		const uint32_t b4 = round16(k.n * 4), b16 = (uint32_t) k.n * 16;
+		const uint32_t a4 = round16(k.na * 4), a16 = (uint32_t) k.na * 16;
+		mbar_arrive_expect_tx(bar, (st.id ? 2 : 1) * (b4 + a4) + b16 + a16);
+		bulk_g2s(buf, st.cell + k.first, b4, bar);
+		bulk_g2s(buf + C * 4, st.ou + k.first, b16, bar);
 		if(st.id)
-			bulk_g2s(buf + C * 20, st.id + first, b4, bar);
+			bulk_g2s(buf + C * 20, st.id + k.first, b4, bar);
+		if(k.na)
+		{
+			bulk_g2s(buf + 4 * k.aslot(), st.cell + k.afirst, a4, bar);
+			bulk_g2s(buf + C * 4 + 16 * k.aslot(), st.ou + k.afirst, a16, bar);
+			if(st.id)
+				bulk_g2s(buf + C * 20 + 4 * k.aslot(), st.id + k.afirst, a4, bar);
+		}
 	}
 
 	template <int C>
@@ -944,8 +974,7 @@ k_push(const __grid_constant__ PushArgs a)
 	const bool ftma = F::field_tma(a, tx0, ty0);
 	const void *Etile = ftma ? F::field_tile(fsm) : F::load_field(a, fsm, W, g.tx, tx0, ty0);
 	// the chunks: the main region's particles, then the arrivals the
-	// previous step left in buffer r; a chunk never spans both, so every
-	// bulk copy starts on a 32-slot boundary
+	// previous step left in buffer r
 	const int r = a.arr_r;
 	const int nm = T.cnt[t];
 	// (a count can pass the capacity: movers that found the region full
@@ -956,20 +985,36 @@ k_push(const __grid_constant__ PushArgs a)
 	const int64_t abase_r = T.abase[t] + (r ? T.abuf1 : 0);
 	const int64_t aofs_w = r ? 0 : T.abuf1;
 	int32_t *const acnt_w = T.acnt[r ^ 1];
+	// with one particle per thread (small tiles) the main region's last,
+	// partial chunk takes arrivals too: a chunk's latency counts there, and
+	// a chunk of arrivals alone is mostly empty (two species 512 x 512, 16
+	// per cell, FP64: 741 us a step in separate chunks, 690 jointly).  With more particles per tile the two extra
+	// instructions per particle cost more than the chunk.
+	constexpr bool kMerge = P == 1;
+	const int nfull = kMerge ? nm / kChunk : 0;
+	const int rem = nm - nfull * kChunk;
+	const int joint = kMerge && rem > 0 ? min(na, kChunk - ((rem + 3) & ~3)) : 0;
 	const int nmc = (nm + kChunk - 1) / kChunk;
-	const int nchunks = nmc + (na + kChunk - 1) / kChunk;
-	auto chunk = [&](int ci, int64_t &first, int &len) {
+	const int nchunks = nmc + (na - joint + kChunk - 1) / kChunk;
+	auto chunk = [&](int ci) {
+		Chunk k;
+		k.na = 0;
+		k.afirst = abase_r;
 		if(ci < nmc)
 		{
-			first = base + (int64_t) ci * kChunk;
-			len = min(kChunk, nm - ci * kChunk);
+			k.first = base + (int64_t) ci * kChunk;
+			k.n = min(kChunk, nm - ci * kChunk);
+			if(kMerge && ci == nfull)
+				k.na = joint;
 		}
 		else
 		{
-			const int o = (ci - nmc) * kChunk;
-			first = abase_r + o;
-			len = min(kChunk, na - o);
+			// joint is all of the arrivals or a multiple of 4
+			const int o = joint + (ci - nmc) * kChunk;
+			k.first = abase_r + o;
+			k.n = min(kChunk, na - o);
 		}
+		return k;
 	};
 	// neighbours are distinct tiles only with at least 3 tiles per side
 	const bool nb_ok = g.ntx >= 3 && g.nty >= 3;
@@ -985,10 +1030,7 @@ k_push(const __grid_constant__ PushArgs a)
 	__syncthreads();
 	if(threadIdx.x == 0 && nchunks > 0)
 	{
-		int64_t f0;
-		int l0;
-		chunk(0, f0, l0);
-		F::template stage_issue<kChunk>(a, s, f0, l0, stage0, &bars[0]);
+		F::template stage_issue<kChunk>(a, s, chunk(0), stage0, &bars[0]);
 	}
 	const int lane = threadIdx.x & 31;
 	if(ftma && !mbar_wait_bounded(&fbar, 0, a.status))
@@ -996,9 +1038,8 @@ k_push(const __grid_constant__ PushArgs a)
 
 	for(int ci = 0; ci < nchunks; ci++)
 	{
-		int64_t cfirst;
-		int clen;
-		chunk(ci, cfirst, clen);
+		const Chunk ck = chunk(ci);
+		const int clen = ck.n + ck.na;
 		if(ci > 0 && ci % kCheckChunks == 0)
 		{
 			// every deposit of the previous chunks precedes the check (and
@@ -1019,10 +1060,7 @@ k_push(const __grid_constant__ PushArgs a)
 			if(ci >= 1 && !mbar_wait_bounded(&ebars[b], ((ci - 1) >> 1) & 1, a.status))
 				s_timeout = 1;
 			fence_proxy_async_smem();
-			int64_t nf;
-			int nl;
-			chunk(ci + 1, nf, nl);
-			F::template stage_issue<kChunk>(a, s, nf, nl, stage0 + b * sb, &bars[b]);
+			F::template stage_issue<kChunk>(a, s, chunk(ci + 1), stage0 + b * sb, &bars[b]);
 		}
 		// this chunk has landed: every global read of the main region's
 		// slots below the end of this chunk is complete, so the in-place
@@ -1043,7 +1081,8 @@ k_push(const __grid_constant__ PushArgs a)
 			const int j = k * kPushThreads + threadIdx.x;
 			const bool valid = j < clen;
 			if(valid)
-				rec[k] = F::template from_stage<kChunk>(buf, j, ids);
+				rec[k] = F::template from_stage<kChunk>(buf,
+						kMerge && j >= ck.n ? j - ck.n + ck.aslot() : j, ids);
 			// the last record is in registers: this warp is done with the
 			// staged chunk, and the buffer goes back to the producer before
 			// the last push, not after it (0.7 % faster on the two-stream
