@@ -444,5 +444,94 @@ CPIC_HD bool pos_split(Pos v, bool neg, int lo_exp, long long &hi, long long &lo
 	return true;
 }
 
+// The cell index and the offset in the cell of position x > 0 from the exact
+// product x idx: i0 = floor(x idx), f = rn(x idx - i0), as one fused
+// multiply-add gives it; false where i0 is out of range or f is 0 or rounds to
+// 1.
+CPIC_HD bool pos_frac(Pos x, Pos idx, int &i0, Pos &f)
+{
+	const uint64_t p = (uint64_t) x.l * idx.l;
+	const uint64_t t = (uint64_t) x.l * idx.h + (uint32_t) (p >> 32);
+	const uint64_t u = (uint64_t) x.h * idx.l + (uint32_t) t;
+	const uint64_t h = (uint64_t) x.h * idx.h + (uint32_t) (t >> 32) + (uint32_t) (u >> 32);
+	const uint64_t l = u << 32 | (uint32_t) p;
+	// the product is (h:l) 2^(e - 127): e + 1 integer bits
+	const int ib = x.e + idx.e + 2;
+	if(ib > 31)
+		return false;
+	uint64_t fh = h, fl = l;
+	int e = ib - 1;
+	i0 = 0;
+	if(ib > 0)
+	{
+		i0 = (int) ((uint32_t) (h >> 32) >> (32 - ib));
+		fh = h << ib | l >> (64 - ib);
+		fl = l << ib;
+		e = -1;
+	}
+	if(fh == 0)
+		return false;
+	const int c = clz64(fh);
+	const uint64_t m = c ? fh << c | fl >> (64 - c) : fh;
+	const uint64_t below = fl << c;
+	f = pos_round((uint32_t) (m >> 32), (uint32_t) m, (uint32_t) (below >> 32) | (uint32_t) below, e - c);
+	return f.e < 0;
+}
+
+// A positive normal float (24 bits: l is 0).
+CPIC_HD bool pos_of(float a, Pos &p)
+{
+#ifdef __CUDA_ARCH__
+	const uint32_t b = __float_as_uint(a);
+#else
+	uint32_t b;
+	std::memcpy(&b, &a, 4);
+#endif
+	const uint32_t f = b >> 23;
+	p.h = b << 8 | 0x80000000u;
+	p.l = 0;
+	p.e = (int) f - 127;
+	return f - 1u < 254u;
+}
+
+// rn(a b) for a of 24 bits (a.l == 0)
+CPIC_HD Pos pos_mul24(Pos a, Pos b)
+{
+	const uint64_t u = (uint64_t) a.h * b.l;
+	const uint64_t h = (uint64_t) a.h * b.h + (uint32_t) (u >> 32);
+	return pos_norm(h, (uint32_t) u, 0u, a.e + b.e + 1);
+}
+
+// a b for a and b of 24 bits: exact in 48
+CPIC_HD Pos pos_mul24x24(Pos a, Pos b)
+{
+	const uint64_t h = (uint64_t) a.h * b.h;
+	const int n = (int) (h >> 63) ^ 1;
+	Pos r;
+	r.h = (uint32_t) ((h << n) >> 32);
+	r.l = (uint32_t) (h << n);
+	r.e = a.e + b.e + 1 - n;
+	return r;
+}
+
+// v rounded to the nearest integer, ties to even, negated when neg; false for
+// v >= 2^62.
+CPIC_HD bool pos_rint(Pos v, bool neg, long long &out)
+{
+	if(v.e >= 62)
+		return false;
+	uint64_t q = 0;
+	if(v.e >= -1)
+	{
+		const int sh = 63 - v.e;                // 2 .. 64 fractional bits
+		const uint64_t m = pos_bits(v);
+		const uint64_t r = sh == 64 ? m : m << (64 - sh);
+		q = sh == 64 ? 0 : m >> sh;
+		q += r > (1ull << 63) - (q & 1ull) ? 1ull : 0ull;
+	}
+	out = neg ? -(long long) q : (long long) q;
+	return true;
+}
+
 } // namespace bits
 } // namespace cpic

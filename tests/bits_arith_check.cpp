@@ -107,6 +107,61 @@ static void check_split(double v, int lo_exp)
 	}
 }
 
+static void check_frac(double x, double idx)
+{
+	Pos p, i, f;
+	int i0 = -1;
+	if(!pos_of(x, p) || !pos_of(idx, i) || !pos_frac(p, i, i0, f))
+		return;
+	checked++;
+	// floor of the exact product: of the rounded one, less one where that
+	// rounded up to an integer
+	double fl = std::floor(x * idx);
+	if(std::fma(x, idx, -fl) < 0.0)
+		fl -= 1.0;
+	const double want = std::fma(x, idx, -fl);
+	if(i0 != (int) fl || !same(pos_val(f), want))
+	{
+		if(bad < 10)
+			std::printf("frac %.17g * %.17g: %d %.17g, want %d %.17g\n", x, idx, i0, pos_val(f), (int) fl, want);
+		bad++;
+	}
+}
+
+static void check_rint(double v)
+{
+	Pos p;
+	long long got;
+	for(int neg = 0; neg < 2; neg++)
+	{
+		if(!pos_of(v, p) || !pos_rint(p, neg != 0, got))
+			continue;
+		checked++;
+		const long long want = std::llrint(neg ? -v : v);
+		if(got != want)
+		{
+			if(bad < 10)
+				std::printf("rint %.17g: %lld, want %lld\n", v, got, want);
+			bad++;
+		}
+	}
+}
+
+static void check_mul24(float a, double b, float c)
+{
+	Pos p, q, r;
+	if(!pos_of(a, p) || !pos_of(c, r) || !pos_of(b, q))
+		return;
+	checked++;
+	const double want = (double) a * b, want2 = (double) a * (double) c;
+	if(!same(pos_val(pos_mul24(p, q)), want) || !same(pos_val(pos_mul24x24(p, r)), want2))
+	{
+		if(bad < 10)
+			std::printf("mul24 %.9g %.17g %.9g\n", a, b, c);
+		bad++;
+	}
+}
+
 // doubles whose products and differences come near ties: few significant
 // bits, runs of ones, a bit at the end
 static double sparse(std::mt19937_64 &rng)
@@ -167,6 +222,28 @@ int main()
 				check_rel(std::ldexp(u(rng), -(int) (rng() % 60)), dx, idx);
 			}
 			check_rel(L, dx, idx);
+		}
+	for(int nx : {4, 16, 64, 128, 256, 4096})
+		for(double L : {6.283185307179586, 1.0, 3.7})
+			for(int k = 0; k < 100000; k++)
+			{
+				const double idx = 1.0 / (L / nx);
+				check_frac((u(rng) - 1.0) * L, idx);
+				check_frac(std::nextafter((double) (rng() % (uint64_t) nx) * (L / nx), (k & 1) ? 1e9 : 0.0), idx);
+				check_frac(std::ldexp(u(rng), -(int) (rng() % 80)), idx);
+			}
+	for(int k = 0; k < 3000000; k++)
+	{
+		check_rint(std::ldexp(u(rng), (int) (rng() % 66) - 4));
+		check_mul24((float) std::ldexp(u(rng), -(int) (rng() % 30)), any(-40, 40) * ((k & 1) ? 1.0 : -1.0),
+				(float) std::ldexp(u(rng), -(int) (rng() % 60)));
+	}
+	for(long long k = 0; k < 5000; k++)
+		for(double d : {0.0, 0.5, 0.25, 0.75})
+		{
+			check_rint((double) k + d);
+			check_rint(std::nextafter((double) k + d, 1e300));
+			check_rint(std::nextafter((double) k + d, 0.0));
 		}
 	const int exps[] = {1, 7, 20, 30, 37, 39, 45, 52, 60, 61, 62};
 	for(long long k = 1; k <= 4096; k++)
