@@ -359,32 +359,31 @@ CPIC_HD Pos pos_mul_int(uint32_t i, Pos b)
 	return pos_norm(h, (uint32_t) u, 0u, 32 - c + b.e);
 }
 
+// v << n and v >> n for 0 <= n < 64 (n is reduced to that where a result is
+// not used).
+CPIC_HD uint64_t shl64(uint64_t v, int n) { return v << (n & 63); }
+CPIC_HD uint64_t shr64(uint64_t v, int n) { return v >> (n & 63); }
+
+// The functions below have no branches where the lanes of a warp would take
+// both sides anyway; where the returned flag is false the other results are
+// meaningless.
+
 // rn(1 - a) for 0 < a < 1 (a.e < 0)
 CPIC_HD Pos pos_one_minus(Pos a)
 {
-	if(a.e == -1)
-	{
-		// a >= 1/2: the difference is exact, in units of 2^-64
-		const uint64_t d = 0ull - pos_bits(a);
-		const int c = clz64(d);
-		const uint64_t m = d << c;
-		Pos r;
-		r.h = (uint32_t) (m >> 32);
-		r.l = (uint32_t) m;
-		r.e = -1 - c;
-		return r;
-	}
-	// a < 1/2: rounded to a multiple of 2^-53, 2^11 of the units.  x:
-	// 2^64 - floor(a 2^64), less one (an odd number, never a tie) when a bit
-	// of a lies below the units
-	const int sh = -1 - a.e;                // 1 ...
+	// in units of 2^-64: x = 2^64 - floor(a 2^64), less one (an odd number,
+	// never a tie) when a bit of a lies below the units.  a >= 1/2 leaves an
+	// exact difference with leading zeros, a < 1/2 a full word to be rounded
+	// to a multiple of 2^11.
+	const int sh = -1 - a.e;                // 0 ...
 	const uint64_t am = pos_bits(a);
-	const uint64_t q = sh < 64 ? am >> sh : 0ull;
-	const bool rest = sh >= 64 || (am << ((64 - sh) & 63)) != 0;
+	const bool far = sh >= 64;
+	const uint64_t q = far ? 0ull : shr64(am, sh);
+	const bool rest = far || shl64(q, sh) != am;
 	const uint64_t x = 0ull - (q | (rest ? 1ull : 0ull));
-	// (x == 0, a below the units with nothing left over, cannot happen: a
-	// shift of 64 or more leaves rest set)
-	return pos_round((uint32_t) (x >> 32), (uint32_t) x, 0u, -1);
+	const int c = clz64(x);
+	const uint64_t m = shl64(x, c);
+	return pos_round((uint32_t) (m >> 32), (uint32_t) m, 0u, -1 - c);
 }
 
 // The cell index and the offset in the cell of position x > 0, as the FP64
@@ -398,21 +397,21 @@ CPIC_HD bool pos_rel(Pos x, Pos dx, Pos idx, int &i0, Pos &rel)
 		return false;
 	uint32_t i = 0;
 	Pos d = x;                              // x - 0 dx
+	// (a branch: the first cell is rare, and selecting between its offset
+	// and the others' took 3 % of the FP64 form's particle kernel)
 	if(p.e >= 0)
 	{
 		i = p.h >> (31 - p.e);
 		const Pos s = pos_mul_int(i, dx);
 		const int k = x.e - s.e;
-		if((unsigned) (k + 1) > 2u)
-			return false;
 		// x is within a factor two of i dx: the difference is exact, in units
 		// of the smaller one's last place
 		const int kx = k > 0 ? 10 : 11, ks = k < 0 ? 10 : 11;
 		const int64_t v = (int64_t) (pos_bits(x) >> kx) - (int64_t) (pos_bits(s) >> ks);
-		if(v <= 0 || (v >> 53) != 0)
+		if((unsigned) (k + 1) > 2u || v <= 0 || (v >> 53) != 0)
 			return false;
 		const int c = clz64((uint64_t) v);
-		const uint64_t m = (uint64_t) v << c;
+		const uint64_t m = shl64((uint64_t) v, c);
 		d.h = (uint32_t) (m >> 32);
 		d.l = (uint32_t) m;
 		d.e = (k > 0 ? s.e : x.e) + 11 - c;
@@ -426,22 +425,20 @@ CPIC_HD bool pos_rel(Pos x, Pos dx, Pos idx, int &i0, Pos &rel)
 // split_fixed, for 1 <= v < 2^62 and 1 <= lo_exp <= 63 (false otherwise).
 CPIC_HD bool pos_split(Pos v, bool neg, int lo_exp, long long &hi, long long &lo)
 {
-	if((unsigned) v.e >= 62u)
-		return false;
 	const int sh = 63 - v.e;                // 2 .. 63 fractional bits of m
 	const uint64_t m = pos_bits(v);
-	const uint64_t q = m >> sh;
-	const uint64_t r = m << (64 - sh);      // the fraction, in units of 2^-64
+	const uint64_t q = shr64(m, sh);
+	const uint64_t r = shl64(m, 64 - sh);   // the fraction, in units of 2^-64
 	// up past one half, or at it from an odd integer
 	const bool up = r > (1ull << 63) - (q & 1ull);
 	const uint64_t f = up ? 0ull - r : r;   // |v - hi|
-	const uint64_t g = f >> (64 - lo_exp);
-	const uint64_t rem = f << lo_exp;
+	const uint64_t g = shr64(f, 64 - lo_exp);
+	const uint64_t rem = shl64(f, lo_exp);
 	const bool up2 = rem > (1ull << 63) - (g & 1ull);
 	const uint64_t h = q + (up ? 1ull : 0ull), l = g + (up2 ? 1ull : 0ull);
 	hi = neg ? -(long long) h : (long long) h;
 	lo = neg != up ? -(long long) l : (long long) l;
-	return true;
+	return (unsigned) v.e < 62u;
 }
 
 // The cell index and the offset in the cell of position x > 0 from the exact
@@ -457,25 +454,17 @@ CPIC_HD bool pos_frac(Pos x, Pos idx, int &i0, Pos &f)
 	const uint64_t l = u << 32 | (uint32_t) p;
 	// the product is (h:l) 2^(e - 127): e + 1 integer bits
 	const int ib = x.e + idx.e + 2;
-	if(ib > 31)
-		return false;
-	uint64_t fh = h, fl = l;
-	int e = ib - 1;
-	i0 = 0;
-	if(ib > 0)
-	{
-		i0 = (int) ((uint32_t) (h >> 32) >> (32 - ib));
-		fh = h << ib | l >> (64 - ib);
-		fl = l << ib;
-		e = -1;
-	}
-	if(fh == 0)
-		return false;
+	const bool some = ib > 0;
+	const int n = some ? ib : 0;
+	i0 = some ? (int) ((uint32_t) (h >> 32) >> ((32 - n) & 31)) : 0;
+	const uint64_t fh = shl64(h, n) | (some ? shr64(l, 64 - n) : 0ull);
+	const uint64_t fl = shl64(l, n);
 	const int c = clz64(fh);
-	const uint64_t m = c ? fh << c | fl >> (64 - c) : fh;
-	const uint64_t below = fl << c;
-	f = pos_round((uint32_t) (m >> 32), (uint32_t) m, (uint32_t) (below >> 32) | (uint32_t) below, e - c);
-	return f.e < 0;
+	const uint64_t m = shl64(fh, c) | (c ? shr64(fl, 64 - c) : 0ull);
+	const uint64_t below = shl64(fl, c);
+	f = pos_round((uint32_t) (m >> 32), (uint32_t) m, (uint32_t) (below >> 32) | (uint32_t) below,
+			(some ? -1 : ib - 1) - c);
+	return (ib <= 31) & (fh != 0) & (f.e < 0);
 }
 
 // A positive normal float (24 bits: l is 0).
@@ -518,19 +507,14 @@ CPIC_HD Pos pos_mul24x24(Pos a, Pos b)
 // v >= 2^62.
 CPIC_HD bool pos_rint(Pos v, bool neg, long long &out)
 {
-	if(v.e >= 62)
-		return false;
-	uint64_t q = 0;
-	if(v.e >= -1)
-	{
-		const int sh = 63 - v.e;                // 2 .. 64 fractional bits
-		const uint64_t m = pos_bits(v);
-		const uint64_t r = sh == 64 ? m : m << (64 - sh);
-		q = sh == 64 ? 0 : m >> sh;
-		q += r > (1ull << 63) - (q & 1ull) ? 1ull : 0ull;
-	}
+	const int sh = 63 - v.e;                // 2 .. 64 fractional bits where v >= 1/2
+	const uint64_t m = pos_bits(v);
+	const bool none = v.e < 0;              // no integer bits
+	const uint64_t q0 = none ? 0ull : shr64(m, sh);
+	const uint64_t r = none ? (v.e == -1 ? m : 0ull) : shl64(m, 64 - sh);
+	const uint64_t q = q0 + (r > (1ull << 63) - (q0 & 1ull) ? 1ull : 0ull);
 	out = neg ? -(long long) q : (long long) q;
-	return true;
+	return v.e < 62;
 }
 
 } // namespace bits

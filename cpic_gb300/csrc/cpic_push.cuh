@@ -205,10 +205,9 @@ struct F64 {
 			bits::Pos w[4], int &i0x, int &i0y)
 	{
 		bits::Pos px, py, rx, ry;
-		bool ok = bits::pos_of(x, px) & bits::pos_of(y, py);
-		ok = ok && bits::pos_rel(px, a.dx_p, a.idx_p, i0x, rx)
-			&& bits::pos_rel(py, a.dx_p, a.idy_p, i0y, ry);
-		if(!ok)
+		const bool ok = bits::pos_of(x, px) & bits::pos_of(y, py);
+		if(!(ok && bits::pos_rel(px, a.dx_p, a.idx_p, i0x, rx)
+				&& bits::pos_rel(py, a.dx_p, a.idy_p, i0y, ry)))
 			return false;
 		const bits::Pos dx = bits::pos_one_minus(rx), dy = bits::pos_one_minus(ry);
 		w[0] = bits::pos_mul(dx, dy);
@@ -278,7 +277,7 @@ struct F64 {
 		for(int pass = 0; ; pass++)
 		{
 			bits::Pos wp[4];
-			bool fast = sp.fast && weights_fast(a, x, y, wp, i0x, i0y);
+			bool fast = weights_fast(a, x, y, wp, i0x, i0y) & (sp.fast != 0);
 			if(pass)
 			{
 				// deposit weights of the new position (interpolate_p2f,
@@ -287,7 +286,7 @@ struct F64 {
 				// (exactly: a power-of-two scale), hi its rounding, and the
 				// remainder c - hi (exact) is kept at 2^m finer resolution.
 				for(int c = 0; c < 4; c++)
-					fast = fast && bits::pos_split(bits::pos_mul(wp[c], sp.qfix_p), sp.qfix_neg != 0,
+					fast &= bits::pos_split(bits::pos_mul(wp[c], sp.qfix_p), sp.qfix_neg != 0,
 							sp.qlo_exp, o.w[c], o.wl[c]);
 				if(!fast)
 				{
@@ -298,8 +297,8 @@ struct F64 {
 				break;
 			}
 			double w[4];
-			fast = fast && bits::pos_normal(wp[0]) && bits::pos_normal(wp[1])
-				&& bits::pos_normal(wp[2]) && bits::pos_normal(wp[3]);
+			fast &= bits::pos_normal(wp[0]) & bits::pos_normal(wp[1])
+				& bits::pos_normal(wp[2]) & bits::pos_normal(wp[3]);
 			if(fast)
 				for(int c = 0; c < 4; c++) w[c] = bits::pos_val(wp[c]);
 			else
