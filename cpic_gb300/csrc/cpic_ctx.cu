@@ -930,8 +930,8 @@ static void fill_species_step(cpic_ctx *c, PushArgs &a, int64_t iter)
 	double dt = iter == 0 ? -p.dt / 2 : p.dt;
 	a.iter = (int) (iter == 0 ? 0 : 1);
 	a.dt = dt;
-	a.cdx_f = (float) (p.dt / c->g.dx);
-	a.cdy_f = (float) (p.dt / c->g.dy);
+	a.cdx_f = iter == 0 ? 0.0f : (float) (p.dt / c->g.dx);
+	a.cdy_f = iter == 0 ? 0.0f : (float) (p.dt / c->g.dy);
 	int64_t chunks = p.plasma_chunks > 0 ? p.plasma_chunks : 1;
 	const bool consts = bits::pos_of(c->g.dx, a.dx_p) & bits::pos_of(c->g.idx, a.idx_p)
 		& bits::pos_of(c->g.idy, a.idy_p);
