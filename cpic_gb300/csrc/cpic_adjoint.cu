@@ -670,7 +670,7 @@ __device__ __forceinline__ void push_one(const AGrid &g, Region &r, const Kick &
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads, 4)
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 8 ? 5 : 4)
 k_push(const __grid_constant__ AGrid g, const Work *work, T *x, T *y, T *ux, T *uy, const T *Ex,
 		const T *Ey, const __grid_constant__ Kick k, T dt, const __grid_constant__ Charge c,
 		unsigned long long *rho, unsigned long long *rsum, T *hx, T *hy)
@@ -934,7 +934,7 @@ __device__ __forceinline__ void kick_back(const Kick &k, T utx, T uty, T &vbx, T
 // rhob = rhob_{j+1}).  par: parity of this step's maxima; the scale comes
 // from the other one's.
 template <typename T>
-__global__ void __launch_bounds__(kThreads, 3)
+__global__ void __launch_bounds__(kThreads, 4)
 k_rev(const __grid_constant__ AGrid g, const Work *work, const T *nx_, const T *ny_, const T *rhob,
 		double c, const T *px_, const T *py_, const T *Ex, const T *Ey, const __grid_constant__ Kick k,
 		T dt, T *pbx, T *pby, T *ubx, T *uby, Scale *sc, int par, double gmax, double n,

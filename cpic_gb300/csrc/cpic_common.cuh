@@ -177,6 +177,14 @@ struct SpillArgs {
 	Spill spill_in[kMaxSpecies];
 };
 
+// Whether the fused kernel takes all species in one launch: while one
+// species' tiles do not fill the GPU.
+constexpr int kSMs = 152;
+inline bool species_together(const PushArgs &a, int ntiles, int per_sm)
+{
+	return a.nspecies > 1 && ntiles < per_sm * kSMs;
+}
+
 // The arguments of species sp moved to index 0 (the fused kernel is
 // launched once per species and reads index 0 only).
 inline PushArgs species_args(const PushArgs &a, int sp)
@@ -551,7 +559,9 @@ inline cudaError_t set_max_dyn_smem(std::initializer_list<const void *> fns, int
 // are left for the caller's cudaGetLastError.
 namespace cpic {
 // ppt: particles per thread of the fused kernel's instance (kPPTChoices)
-cudaError_t launch_push_f64(const PushArgs &a, int ntiles, size_t smem, int ppt, cudaStream_t s);
+// per_sm: resident blocks per SM of that instance (the function below it)
+cudaError_t launch_push_f64(const PushArgs &a, int ntiles, size_t smem, int ppt, int per_sm,
+		cudaStream_t s);
 int push_f64_blocks_per_sm(size_t smem, int ppt);
 void launch_spill_f64(const SpillArgs &a, cudaStream_t s);
 // What the field stage's last kernel clears for the next particle stage:
@@ -571,7 +581,8 @@ cudaError_t launch_poisson_f64(const Grid &g, const long long *rho, double qinv,
 		double2 *spec, const double2 *twx, const double2 *twy, double *phi, cudaStream_t s,
 		const long long *rho_lo, double qinv_lo, const double *Gt);
 
-cudaError_t launch_push_mix(const PushArgs &a, int ntiles, size_t smem, int ppt, cudaStream_t s);
+cudaError_t launch_push_mix(const PushArgs &a, int ntiles, size_t smem, int ppt, int per_sm,
+		cudaStream_t s);
 // resident blocks per SM of the mixed fused kernel at this dynamic shared
 // memory, for a store with or without ids (0 on error)
 int push_mix_blocks_per_sm(size_t smem, bool ids, int ppt, bool gp2);

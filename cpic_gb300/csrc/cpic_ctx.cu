@@ -65,6 +65,7 @@ struct cpic_ctx {
 	cudaStream_t stream;
 	int order_mode;           // tile order: 0 undecided, 1 recomputed, 2 kept
 	unsigned order_tick;      // steps since the layout was made
+	int push_per_sm;          // resident blocks per SM of the fused kernel (0: not asked yet)
 	int nspecies;
 	SpeciesHost sp[kMaxSpecies];
 	// parity of the double-buffered spill lists and arrivals buffers: the
@@ -731,6 +732,8 @@ __global__ void k_field_energy(Grid g, const double *Ex, const double *Ey, const
 		const long long *rho, double *part)
 {
 	__shared__ double sh[2][256];
+	pdl_trigger();
+	pdl_wait();
 	int iy = blockIdx.x;
 	double e = 0.0;
 	long long q = 0;
@@ -1392,13 +1395,22 @@ static int rebuild_if_spilled(cpic_ctx *c, bool all = true, bool *rebuilt = null
 	return CPIC_OK;
 }
 
+// ctl into the pinned copy: a dependent launch where a copy by the engine
+// would follow (it starts while the step's last kernel drains).
+__global__ void k_probe(const int32_t *ctl, int32_t *out)
+{
+	pdl_wait();
+	if(threadIdx.x < kCtl)
+		out[threadIdx.x] = ctl[threadIdx.x];
+}
+
 // After a particle stage: the status word and the spill counts in one round
 // trip (pinned host copies, one synchronisation); a rebuild only when a
 // spill list has grown past its threshold.
 static int step_check(cpic_ctx *c)
 {
 	cudaStream_t st = c->stream;
-	CK(cudaMemcpyAsync(c->probe_h, c->ctl, kCtl * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+	CK(launch_pdl(k_probe, 1, 32, 0, st, c->ctl, c->probe_h));
 	CK(cudaStreamSynchronize(st));
 	const int32_t *counts = c->probe_h + (spill_count(c, c->spill_cur, 0) - c->ctl);
 	const uint32_t sw = (uint32_t) c->probe_h[0];
@@ -1421,18 +1433,13 @@ static int step_check(cpic_ctx *c)
 // Whether ordering the tiles can shorten the fused kernel: only when its
 // blocks do not all fit on the GPU at once (more than one wave), and the
 // layout is small enough for the one-block sort.
-static bool tile_order_pays(const cpic_ctx *c, size_t smem)
+static bool tile_order_pays(const cpic_ctx *c)
 {
 	if(c->ntiles > kOrderMaxTiles)
 		return false;
-	int dev = 0, nsm = 0;
-	if(cudaGetDevice(&dev) != cudaSuccess
-			|| cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-		return true;
-	const int per_sm = c->precision == CPIC_MIXED
-		? push_mix_blocks_per_sm(smem, c->p.track_ids != 0, c->ppt, c->g.pow2 != 0)
-		: push_f64_blocks_per_sm(smem, c->ppt);
-	return per_sm <= 0 || (int64_t) c->ntiles > (int64_t) per_sm * nsm;
+	const int64_t blocks = (int64_t) c->ntiles
+		* (c->ntiles < c->push_per_sm * kSMs ? c->nspecies : 1);
+	return c->push_per_sm <= 0 || blocks > (int64_t) c->push_per_sm * kSMs;
 }
 
 // One fused particle stage (gather, push, re-bin, deposit) without
@@ -1486,16 +1493,20 @@ static int plasma_stage_async(cpic_ctx *c, bool deposit_only, cudaEvent_t ev0 = 
 		launch_spill_f64(sa, st);
 	c->spill_empty = false;
 	if(ev0) CK(cudaEventRecord(ev0, st));
+	if(!c->push_per_sm)
+		c->push_per_sm = c->precision == CPIC_MIXED
+			? push_mix_blocks_per_sm(smem, c->p.track_ids != 0, c->ppt, c->g.pow2 != 0)
+			: push_f64_blocks_per_sm(smem, c->ppt);
 	if(c->precision == CPIC_MIXED)
-		CK(launch_push_mix(sa.p, c->ntiles, smem, c->ppt, st));
+		CK(launch_push_mix(sa.p, c->ntiles, smem, c->ppt, c->push_per_sm, st));
 	else
-		CK(launch_push_f64(sa.p, c->ntiles, smem, c->ppt, st));
+		CK(launch_push_f64(sa.p, c->ntiles, smem, c->ppt, c->push_per_sm, st));
 	if(ev1) CK(cudaEventRecord(ev1, st));
 	CK(cudaGetLastError());
 	// the next launch's tile order, from the main regions' counts and the
 	// arrivals this launch left for it
 	if(c->order_mode == 0)
-		c->order_mode = tile_order_pays(c, smem) ? 1 : 2;
+		c->order_mode = tile_order_pays(c) ? 1 : 2;
 	// every kOrderEvery steps: the counts move slowly against the order's
 	// classes (a sixteenth of the mean), and any order is a valid one
 	if(c->order_mode == 1 && c->order_tick++ % kOrderEvery == 0)
@@ -1923,6 +1934,7 @@ CPIC_API int cpic_add_species(cpic_ctx_t *c, double q, double m, int64_t n,
 		}
 		c->g.halo = H;
 	}
+	c->push_per_sm = 0;
 	return s;
 }
 
@@ -2240,13 +2252,12 @@ CPIC_API int cpic_field_energy(cpic_ctx_t *c, double *out)
 {
 	if(!c || !out) return CPIC_EINVAL;
 	int ny = c->g.ny;
-	int r = ensure_scratch(c, 2 * (size_t) ny);
-	if(r) return r;
 	cudaStream_t st = c->stream;
 	const double *h = c->part_h;
-	k_field_energy<<<ny, 256, 0, st>>>(c->g, c->Ex64, c->Ey64,
-			c->precision == CPIC_MIXED ? c->E32 : nullptr, c->rho, c->scratch);
-	CK(cudaMemcpyAsync(c->part_h, c->scratch, 2 * ny * sizeof(double), cudaMemcpyDeviceToHost, st));
+	// the rows' sums straight into the pinned buffer: a copy after the kernel
+	// is one more dependent operation in a call that is all latency
+	CK(launch_pdl(k_field_energy, ny, 256, 0, st, c->g, c->Ex64, c->Ey64,
+			c->precision == CPIC_MIXED ? c->E32 : nullptr, c->rho, c->part_h));
 	CK(cudaStreamSynchronize(st));
 	double we = 0.0, q = 0.0;
 	for(int i = 0; i < ny; i++) { we += h[2 * i]; q += h[2 * i + 1]; }

@@ -99,7 +99,8 @@ static const void *push_f64_fn(int P)
 static cudaError_t push_f64_attrs()
 {
 	return g_push_f64_once.run([] {
-		return set_max_dyn_smem({push_f64_fn(1), push_f64_fn(2), push_f64_fn(4)}, 200 * 1024, true);
+		return set_max_dyn_smem({push_f64_fn(1), push_f64_fn(2), push_f64_fn(4),
+				(const void *) k_push<F64, F64::min_blocks(1), true, 1, true, true>}, 200 * 1024, true);
 	});
 }
 
@@ -114,11 +115,15 @@ int push_f64_blocks_per_sm(size_t smem, int ppt)
 	return b;
 }
 
-cudaError_t launch_push_f64(const PushArgs &a, int ntiles, size_t smem, int ppt, cudaStream_t s)
+cudaError_t launch_push_f64(const PushArgs &a, int ntiles, size_t smem, int ppt, int per_sm,
+		cudaStream_t s)
 {
 	if(!ppt_supported(ppt)) return cudaErrorInvalidValue;
 	cudaError_t e = push_f64_attrs();
 	if(e != cudaSuccess) return e;
+	if(ppt == 1 && species_together(a, ntiles, per_sm))
+		return launch_pdl(k_push<F64, F64::min_blocks(1), true, 1, true, true>, dim3(ntiles, a.nspecies),
+				kPushThreads, smem, s, a);
 	for(int sp = 0; sp < a.nspecies; sp++)
 	{
 		const PushArgs b = species_args(a, sp);

@@ -143,6 +143,20 @@ static const void *push_mix_fn(bool hi, bool ids, int P, bool gp2)
 		: push_mix_fn_p<2>(hi, ids, gp2);
 }
 
+// All species in one launch: the register-capped instances with 1 and 2
+// particles per thread.
+typedef void (*PushKernel)(const PushArgs);
+template <int P, bool G>
+static PushKernel push_mix_all_pg(bool ids)
+{
+	return ids ? k_push<Mix, Mix::kHiBlocks, true, P, G, true> : k_push<Mix, Mix::kHiBlocks, false, P, G, true>;
+}
+static PushKernel push_mix_all(bool ids, int P, bool gp2)
+{
+	if(P == 1) return gp2 ? push_mix_all_pg<1, true>(ids) : push_mix_all_pg<1, false>(ids);
+	return gp2 ? push_mix_all_pg<2, true>(ids) : push_mix_all_pg<2, false>(ids);
+}
+
 static cudaError_t push_mix_attrs()
 {
 	return g_push_mix_once.run([] {
@@ -153,6 +167,11 @@ static cudaError_t push_mix_attrs()
 					for(int gp2 = 0; gp2 < 2 && e == cudaSuccess; gp2++)
 						e = set_max_dyn_smem({push_mix_fn(hi != 0, ids != 0, P, gp2 != 0)},
 								200 * 1024, true);
+		for(int P = 1; P <= 2; P++)
+			for(int ids = 0; ids < 2 && e == cudaSuccess; ids++)
+				for(int gp2 = 0; gp2 < 2 && e == cudaSuccess; gp2++)
+					e = set_max_dyn_smem({(const void *) push_mix_all(ids != 0, P, gp2 != 0)},
+							200 * 1024, true);
 		return e;
 	});
 }
@@ -207,16 +226,20 @@ static void launch_push_mix_p(const PushArgs &b, int ntiles, size_t smem, bool h
 	else launch_push_mix_pg<P, false>(b, ntiles, smem, hi, ids, s);
 }
 
-cudaError_t launch_push_mix(const PushArgs &a, int ntiles, size_t smem, int ppt, cudaStream_t s)
+cudaError_t launch_push_mix(const PushArgs &a, int ntiles, size_t smem, int ppt, int per_sm,
+		cudaStream_t s)
 {
 	if(!ppt_supported(ppt)) return cudaErrorInvalidValue;
 	cudaError_t e = push_mix_attrs();
 	if(e != cudaSuccess) return e;
+	const bool hi = per_sm >= Mix::kHiBlocks;
+	if(hi && ppt <= 2 && species_together(a, ntiles, per_sm))
+		return launch_pdl(push_mix_all(a.mix[0].id != nullptr, ppt, a.g.pow2 != 0),
+				dim3(ntiles, a.nspecies), kPushThreads, smem, s, a);
 	for(int sp = 0; sp < a.nspecies; sp++)
 	{
 		const PushArgs b = species_args(a, sp);
 		const bool ids = b.mix[0].id != nullptr;
-		const bool hi = push_mix_hi(smem, ids, ppt, b.g.pow2 != 0);
 		if(ppt == 1) launch_push_mix_p<1>(b, ntiles, smem, hi, ids, s);
 		else if(ppt == 4) launch_push_mix_p<4>(b, ntiles, smem, hi, ids, s);
 		else launch_push_mix_p<2>(b, ntiles, smem, hi, ids, s);
