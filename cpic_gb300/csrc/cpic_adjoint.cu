@@ -494,7 +494,6 @@ k_deposit(const __grid_constant__ AGrid g, const Work *work, const T *x, const T
 		const __grid_constant__ Charge c, unsigned long long *rho, unsigned long long *rsum)
 {
 	extern __shared__ uint32_t smem[];
-	pdl_trigger();
 	pdl_wait();
 	const Work w = work[blockIdx.x];
 	if(w.tile < 0) return;
@@ -518,7 +517,6 @@ k_deposit(const __grid_constant__ AGrid g, const Work *work, const T *x, const T
 template <typename T>
 __global__ void k_E(AGrid g, const T *phi, T *Ex, T *Ey, long long *rho, long long *rsum)
 {
-	pdl_trigger();
 	pdl_wait();
 	int64_t ng = (int64_t) g.nx * g.ny;
 	T cx = (T) (0.5 * g.idx), cy = (T) (0.5 * g.idy);
@@ -676,7 +674,6 @@ k_push(const __grid_constant__ AGrid g, const Work *work, T *x, T *y, T *ux, T *
 		unsigned long long *rho, unsigned long long *rsum, T *hx, T *hy)
 {
 	extern __shared__ uint32_t smem[];
-	pdl_trigger();
 	pdl_wait();
 	const Work w = work[blockIdx.x];
 	if(w.tile < 0) return;
@@ -751,7 +748,6 @@ __global__ void k_loss_grad(int64_t ng, const T *Ex, const T *Ey, double f, T *E
 template <typename T>
 __global__ void k_div(AGrid g, const T *Ebx, const T *Eby, const long long *fix, Scale *sc, T *phib)
 {
-	pdl_trigger();
 	pdl_wait();
 	int64_t ng = (int64_t) g.nx * g.ny;
 	T cx = (T) (0.5 * g.idx), cy = (T) (0.5 * g.idy);
@@ -785,7 +781,6 @@ template <typename T>
 __global__ void k_absmax(int64_t ng, const T *v, Scale *sc, long long *fix, int par)
 {
 	__shared__ unsigned long long sh[kThreads / 32];
-	pdl_trigger();
 	pdl_wait();
 	if(blockIdx.x == 0 && threadIdx.x == 0) { sc->u[par] = 0; sc->p[par] = 0; }
 	unsigned long long m = 0;
@@ -943,7 +938,6 @@ k_rev(const __grid_constant__ AGrid g, const Work *work, const T *nx_, const T *
 	extern __shared__ uint32_t smem[];
 	__shared__ unsigned long long sh[kThreads / 32];
 	__shared__ int s_eexp;
-	pdl_trigger();
 	pdl_wait();
 	const Work w = work[blockIdx.x];
 	// (block 0 leaves the scale for k_div even without work of its own)
@@ -1428,9 +1422,9 @@ CPIC_API int cpic_adj_create(const cpic_adj_params_t *p, int64_t n, cpic_adj_t *
 		cudaMemcpy(cosx, cx.data(), p->nx * sizeof(double), cudaMemcpyHostToDevice);
 		cudaMemcpy(cosy, cy.data(), p->ny * sizeof(double), cudaMemcpyHostToDevice);
 		if(a->f64) k_green<double><<<blocks_for(nh * p->ny), 256>>>(a->g.nx, a->g.ny, cosx, cosy,
-				P<double>(a->green));
+				P<double>(a->green), green_scale<double>(a->g.nx, a->g.ny));
 		else k_green<float><<<blocks_for(nh * p->ny), 256>>>(a->g.nx, a->g.ny, cosx, cosy,
-				P<float>(a->green));
+				P<float>(a->green), green_scale<float>(a->g.nx, a->g.ny));
 		for(int dim = 0; dim < 2; dim++)
 		{
 			int64_t m = dim == 0 ? p->nx : p->ny;

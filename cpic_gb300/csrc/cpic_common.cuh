@@ -359,20 +359,24 @@ warp_reserve(int32_t *cnt, bool move, int dest)
 // ------------------------------------- dependent launches in one stream
 //
 // The kernels of a step depend on each other in a chain.  They are launched
-// with programmatic stream serialisation (launch_pdl): a kernel's blocks may
-// start while its predecessor drains, run what touches no data of the
-// chain (shared-memory set-up, constant tables), and wait for the
-// predecessor's completion and memory in pdl_wait().  Every thread of such a
-// kernel calls pdl_wait() before its first access to such data, so a
-// kernel's completion implies that of all before it.  Measured on empty
-// kernels: 1.4 us per dependent launch instead of 3.1.
+// with programmatic stream serialisation (launch_pdl): a kernel is made ready
+// while its predecessor runs, and its blocks wait for the predecessor's
+// completion and memory in pdl_wait().  Every thread of such a kernel calls
+// pdl_wait() before its first access to data of the chain, so a kernel's
+// completion implies that of all before it.  Measured on empty kernels: 1.4
+// us per dependent launch instead of 3.1.
 __device__ __forceinline__ void pdl_wait()
 {
 	asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// Lets the next kernel's blocks start once every block of this one has got
-// here.
+// Lets the next kernel's blocks start, and run what touches no data of the
+// chain, once every block of this one has got here; without it they start
+// when this one's blocks are done.  Only in kernels that leave the SMs
+// nearly empty (the spill pass, the tile order): next to a working kernel the
+// early blocks go where there is room, not where they will run best, and
+// stay there (a 512 x 512 FP64 solve, one or two blocks per SM and kernel: 99
+// us with triggers everywhere, 58 without; 250 x 150 FP64 step 168 and 140).
 __device__ __forceinline__ void pdl_trigger()
 {
 	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -732,7 +732,6 @@ __global__ void k_field_energy(Grid g, const double *Ex, const double *Ey, const
 		const long long *rho, double *part)
 {
 	__shared__ double sh[2][256];
-	pdl_trigger();
 	pdl_wait();
 	int iy = blockIdx.x;
 	double e = 0.0;
@@ -1726,7 +1725,8 @@ CPIC_API int cpic_create(const cpic_params_t *p, cpic_ctx_t **out)
 			r = CPIC_ENOMEM;
 			goto fail;
 		}
-		k_green<double><<<grid_blocks(nh * g.ny), 256>>>(g.nx, g.ny, c->cosx, c->cosy, c->green64);
+		k_green<double><<<grid_blocks(nh * g.ny), 256>>>(g.nx, g.ny, c->cosx, c->cosy, c->green64,
+				green_scale<double>(g.nx, g.ny));
 	}
 	else
 	{
@@ -1735,7 +1735,8 @@ CPIC_API int cpic_create(const cpic_params_t *p, cpic_ctx_t **out)
 			r = CPIC_ENOMEM;
 			goto fail;
 		}
-		k_green<float><<<grid_blocks(nh * g.ny), 256>>>(g.nx, g.ny, c->cosx, c->cosy, c->green32);
+		k_green<float><<<grid_blocks(nh * g.ny), 256>>>(g.nx, g.ny, c->cosx, c->cosy, c->green32,
+				green_scale<float>(g.nx, g.ny));
 	}
 	if(cudaDeviceSynchronize() != cudaSuccess) { r = CPIC_ECUDA; goto fail; }
 	*out = c;

@@ -482,6 +482,18 @@ __device__ __forceinline__ const C *fft_tw_stage(C *dst, const C *tw, int n, boo
 	return dst;
 }
 
+// The FP64 form keeps scalings by powers of two out of its transforms (their
+// multiplications were 5 % of the row kernels, which the FP64 pipe bounds):
+// the half of the row split, and 1 / (nx ny) where that is one, are folded
+// into the Green's function, exactly.  FP32 multiplies where it always did.
+template <typename T>
+inline double green_scale(int nx, int ny)
+{
+	if(sizeof(T) == 4) return 1.0;
+	const bool pow2 = (nx & (nx - 1)) == 0 && (ny & (ny - 1)) == 0;
+	return pow2 ? 0.5 / ((double) nx * (double) ny) : 0.5;
+}
+
 // The number of grid nodes, to divide by: N, 1 / N (rounded) and whether N is
 // a power of two (then v * r is v / N exactly).
 template <typename T>
@@ -508,15 +520,25 @@ __device__ __forceinline__ double over(double v, const NodeCount<double> &c)
 	return c.pow2 ? v * c.r : bits::div_by(v, c.n, c.r);
 }
 
+// phi from the inverse transform (green_scale may have divided already)
+__device__ __forceinline__ float phi_of(float v, const NodeCount<float> &c) { return over(v, c); }
+__device__ __forceinline__ double phi_of(double v, const NodeCount<double> &c)
+{
+	return c.pow2 ? v : bits::div_by(v, c.n, c.r);
+}
+
 // The kernels below are static: the FP64 units (built without FMA
 // contraction) and the mixed and adjoint units (built with it) each get their
 // own copy, so a launch always runs the device code of the unit that makes
 // it, and a kernel attribute set in one unit leaves the other units' kernels
 // alone.
 
-// The two half spectra of a transformed row pair.
-template <typename C, typename T>
-__device__ __forceinline__ void split_rows(const C *Z, int nx, int nh, C *spec, int r0, bool two, T half)
+// The two half spectra of a transformed row pair, FP64: twice them
+// (green_scale).
+__device__ __forceinline__ float half_of(float v) { return v * 0.5f; }
+__device__ __forceinline__ double half_of(double v) { return v; }
+template <typename C>
+__device__ __forceinline__ void split_rows(const C *Z, int nx, int nh, C *spec, int r0, bool two)
 {
 	for(int k = threadIdx.x; k < nh; k += blockDim.x)
 	{
@@ -524,11 +546,11 @@ __device__ __forceinline__ void split_rows(const C *Z, int nx, int nh, C *spec, 
 		C q = Z[k == 0 ? 0 : nx - k];
 		q.y = -q.y;                          // conj(Z[-k])
 		C A, B;
-		A.x = (p.x + q.x) * half;
-		A.y = (p.y + q.y) * half;
+		A.x = half_of(p.x + q.x);
+		A.y = half_of(p.y + q.y);
 		// (p - q) / (2i) = -i (p - q) / 2
-		B.x = (p.y - q.y) * half;
-		B.y = -(p.x - q.x) * half;
+		B.x = half_of(p.y - q.y);
+		B.y = half_of(-(p.x - q.x));
 		spec[(int64_t) r0 * nh + k] = A;
 		if(two) spec[(int64_t) (r0 + 1) * nh + k] = B;
 	}
@@ -554,7 +576,6 @@ static __global__ void k_rows_fwd(const __grid_constant__ FftPlan px, int ny, co
 	const int nx = px.n;
 	C *a = reinterpret_cast<C *>(smem_raw);
 	C *b = a + nx;
-	pdl_trigger();
 	tw = fft_tw_stage(b + nx, tw, fft_tw_elems(px), tw_sm);
 	pdl_wait();
 	int r0 = 2 * blockIdx.x;
@@ -583,15 +604,15 @@ static __global__ void k_rows_fwd(const __grid_constant__ FftPlan px, int ny, co
 	}
 	__syncthreads();
 	const C *Z = fft_any<C>(a, b, px, 1, nx, -1, tw);
-	split_rows(Z, nx, nh, spec, r0, two, (T) 0.5);
+	split_rows(Z, nx, nh, spec, r0, two);
 }
 
 // The Green's function G(kx, ky) = 1 / (2 (cos(2 pi kx/nx) + cos(2 pi
 // ky/ny)) - 4), G(0, 0) = 0 (solver.c:269-280), stored once per context in
 // column order Gt[kx * ny + ky] (the order k_cols reads it), as type T.
-// Evaluated in FP64 from the cosine tables.
+// Evaluated in FP64 from the cosine tables, times scale (green_scale).
 template <typename T>
-static __global__ void k_green(int nx, int ny, const double *cosx, const double *cosy, T *Gt)
+static __global__ void k_green(int nx, int ny, const double *cosx, const double *cosy, T *Gt, double scale)
 {
 	int nh = nx / 2 + 1;
 	int64_t total = (int64_t) nh * ny;
@@ -599,7 +620,7 @@ static __global__ void k_green(int nx, int ny, const double *cosx, const double 
 			i += (int64_t) gridDim.x * blockDim.x)
 	{
 		int kx = (int) (i / ny), row = (int) (i - (int64_t) kx * ny);
-		double G = (kx == 0 && row == 0) ? 0.0 : 1.0 / (2.0 * (cosx[kx] + cosy[row]) - 4.0);
+		double G = (kx == 0 && row == 0) ? 0.0 : scale / (2.0 * (cosx[kx] + cosy[row]) - 4.0);
 		Gt[i] = (T) G;
 	}
 }
@@ -617,7 +638,6 @@ __device__ __forceinline__ void cols_body(const FftPlan &py, int nh, int cb, typ
 	const int pitch = fft_pitch(ny, cb);
 	C *a = reinterpret_cast<C *>(smem_raw);
 	C *b = a + (size_t) cb * pitch;
-	pdl_trigger();
 	tw = fft_tw_stage(b + (size_t) cb * pitch, tw, fft_tw_elems(py), tw_sm, twsh);
 	pdl_wait();
 	// element idx of the block's columns: row idx / ncol, column idx % ncol
@@ -672,7 +692,6 @@ static __global__ void k_rows_inv(const __grid_constant__ FftPlan px, int ny,
 	const int nx = px.n;
 	C *a = reinterpret_cast<C *>(smem_raw);
 	C *b = a + nx;
-	pdl_trigger();
 	tw = fft_tw_stage(b + nx, tw, fft_tw_elems(px), tw_sm, twsh);
 	pdl_wait();
 	int r0 = 2 * blockIdx.x;
@@ -704,8 +723,8 @@ static __global__ void k_rows_inv(const __grid_constant__ FftPlan px, int ny,
 	for(int i = threadIdx.x; i < nx; i += blockDim.x)
 	{
 		C v = Y[i];
-		phi[(int64_t) r0 * nx + i] = over(v.x, N);
-		if(two) phi[(int64_t) (r0 + 1) * nx + i] = over(v.y, N);
+		phi[(int64_t) r0 * nx + i] = phi_of(v.x, N);
+		if(two) phi[(int64_t) (r0 + 1) * nx + i] = phi_of(v.y, N);
 	}
 }
 
@@ -721,7 +740,6 @@ static __global__ void k_rows_fwd_real(const __grid_constant__ FftPlan px, int n
 	const int nx = px.n;
 	C *a = reinterpret_cast<C *>(smem_raw);
 	C *b = a + nx;
-	pdl_trigger();
 	tw = fft_tw_stage(b + nx, tw, fft_tw_elems(px), tw_sm, twsh);
 	pdl_wait();
 	int r0 = 2 * blockIdx.x;
@@ -736,7 +754,7 @@ static __global__ void k_rows_fwd_real(const __grid_constant__ FftPlan px, int n
 	}
 	__syncthreads();
 	const C *Z = fft_any<C>(a, b, px, 1, nx, -1, tw);
-	split_rows(Z, nx, nh, spec, r0, two, (T) 0.5);
+	split_rows(Z, nx, nh, spec, r0, two);
 }
 
 // ----------------------------------------------------------------- launch

@@ -17,7 +17,6 @@ namespace cpic {
 __global__ void k_E_f64(Grid g, const double *phi, double *Ex, double *Ey, double rdx2, double rdy2,
 		const NextStage next)
 {
-	pdl_trigger();
 	pdl_wait();
 	clear_counts(next);
 	double dx2 = 2 * g.dx, dy2 = 2 * g.dy;

@@ -13,7 +13,6 @@ namespace cpic {
 // over blockIdx.y, so no index is divided.
 __global__ void k_E_mix(Grid g, const float *phi, float2 *E, const NextStage next)
 {
-	pdl_trigger();
 	pdl_wait();
 	clear_counts(next);
 	// four nodes of one row per thread (nx a multiple of 4): one float4 of
@@ -53,7 +52,6 @@ __global__ void k_E_mix(Grid g, const float *phi, float2 *E, const NextStage nex
 // The same for any nx: one node per thread.
 __global__ void k_E_mix_any(Grid g, const float *phi, float2 *E, const NextStage next)
 {
-	pdl_trigger();
 	pdl_wait();
 	clear_counts(next);
 	const float rdx2 = (float) (1.0 / (2 * g.dx)), rdy2 = (float) (1.0 / (2 * g.dy));

@@ -71,14 +71,14 @@ __device__ __forceinline__ double cos_of(const double2 *tw, int j, int log2n)
 // table): G(kx, ky) is even in ky, so each block divides for half of its
 // rows, into shared memory behind the transform's buffers.
 __global__ void k_noalloc_cols(const __grid_constant__ FftPlan py, int nh, int log2nx, double2 *spec,
-		const double2 *tw, size_t buf_bytes)
+		const double2 *tw, size_t buf_bytes, double scale)
 {
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	double *gs = reinterpret_cast<double *>(smem_raw + buf_bytes);
 	const int kx = blockIdx.x, ny = py.n;
 	const double cx = cos_of(tw, kx, log2nx);
 	for(int row = threadIdx.x; row <= ny / 2; row += blockDim.x)
-		gs[row] = (kx == 0 && row == 0) ? 0.0 : 1.0 / (2.0 * (cx + cos_of(tw, row, py.log2n)) - 4.0);
+		gs[row] = (kx == 0 && row == 0) ? 0.0 : scale / (2.0 * (cx + cos_of(tw, row, py.log2n)) - 4.0);
 	cols_body<double>(py, nh, 1, spec, tw, kLog2MaxN - py.log2n, true, smem_raw,
 			[=](int, int row) { return gs[2 * row <= ny ? row : ny - row]; });
 }
@@ -90,9 +90,10 @@ __global__ void k_noalloc_cols(const __grid_constant__ FftPlan py, int nh, int l
 // since calls that overlap on the GPU are the caller's to serialise.  A
 // device is marked ready only when every step succeeded, so a failed set-up
 // is retried by the next call; a table launch that was only recorded into a
-// graph does not count.
-static int scratch_for_current_device(void **out, cudaStream_t s)
+// graph does not count.  *first: this call launched the table.
+static int scratch_for_current_device(void **out, cudaStream_t s, bool *first)
 {
+	*first = false;
 	int dev = -1;
 	if(cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices)
 		return CPIC_ENODEV;
@@ -116,6 +117,7 @@ static int scratch_for_current_device(void **out, cudaStream_t s)
 	}
 	if(!g_tables_ready[dev])
 	{
+		*first = true;
 		cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
 		double2 *tw = (double2 *) g_scratch_addr[dev] + kSpecElems;
 		void *argv[] = {&tw};
@@ -151,7 +153,8 @@ cpic_poisson_noalloc(const double *rho, double *phi, int64_t nx, int64_t ny, voi
 	}
 	void *base = nullptr;
 	cudaStream_t s = (cudaStream_t) stream;
-	int r = scratch_for_current_device(&base, s);
+	bool first;                     // the table was launched by this call
+	int r = scratch_for_current_device(&base, s, &first);
 	if(r) return r;
 	double2 *spec = (double2 *) base;
 	const double2 *tw = spec + kSpecElems;
@@ -162,18 +165,31 @@ cpic_poisson_noalloc(const double *rho, double *phi, int64_t nx, int64_t ny, voi
 
 	// one column per block, at most 257 of them
 	// (each launch reports its own error, not an earlier one left pending on
-	// the thread).  The first one waits for whatever the caller has queued in
-	// the ordinary way: that may be any operation, or the table's launch.
-	double2 *spec0 = spec;
-	bool kept = true;
-	int nyarg = nyi, sharg = sx;
-	FftPlan pxarg = px;
-	void *argv[] = {&pxarg, &nyarg, (void *) &rho, &spec0, (void *) &tw, &kept, &sharg};
-	cudaError_t e = cudaLaunchKernel((const void *) k_rows_fwd_real<double>, dim3(nyi / 2),
-			dim3(rs.threads), argv, rs.smem, s);
+	// the thread).  All three are dependent launches: the first waits on the
+	// device for whatever the caller has queued.  In a capture, where its
+	// predecessors may be any nodes, and behind the table's launch, whose
+	// result it reads early, the first one is an ordinary launch.
+	cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+	cudaError_t e = first ? cudaSuccess : cudaStreamIsCapturing(s, &cap);
+	if(e == cudaSuccess)
+	{
+		if(cap == cudaStreamCaptureStatusNone)
+			e = launch_pdl(k_rows_fwd_real<double>, nyi / 2, rs.threads, rs.smem, s, px, nyi, rho, spec, tw,
+					true, sx);
+		else
+		{
+			double2 *spec0 = spec;
+			bool kept = true;
+			int nyarg = nyi, sharg = sx;
+			FftPlan pxarg = px;
+			void *argv[] = {&pxarg, &nyarg, (void *) &rho, &spec0, (void *) &tw, &kept, &sharg};
+			e = cudaLaunchKernel((const void *) k_rows_fwd_real<double>, dim3(nyi / 2), dim3(rs.threads),
+					argv, rs.smem, s);
+		}
+	}
 	if(e == cudaSuccess)
 		e = launch_pdl(k_noalloc_cols, nh, cs.threads, cs.smem + (nyi / 2 + 1) * sizeof(double), s, py, nh,
-				px.log2n, spec, tw, cs.smem);
+				px.log2n, spec, tw, cs.smem, green_scale<double>(nxi, nyi));
 	if(e == cudaSuccess)
 		e = launch_pdl(k_rows_inv<double>, nyi / 2, rs.threads, rs.smem, s, px, nyi, spec, tw, phi, true,
 				node_count<double>(nxi, nyi), sx);

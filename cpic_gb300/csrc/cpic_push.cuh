@@ -951,7 +951,6 @@ k_push(const __grid_constant__ PushArgs a)
 	unsigned char *fsm = stage0 + 2 * sb;
 
 	// barriers set up while the previous kernel drains
-	pdl_trigger();
 	if(threadIdx.x == 0)
 	{
 		s_cursor = 0;
