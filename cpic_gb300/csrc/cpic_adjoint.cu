@@ -1361,8 +1361,14 @@ CPIC_API int cpic_adj_create(const cpic_adj_params_t *p, int64_t n, cpic_adj_t *
 	a->nckpt = (int) ((p->nsteps + K - 1) / K);
 	a->idx_ok = bits::pos_of(a->g.idx, a->g.idx_p) & bits::pos_of(a->g.idy, a->g.idy_p);
 	// Particles per block: enough blocks for the SMs to finish together (four
-	// are resident on each), else as many as amortise the region's flush.
-	a->chunk = n >= 4 << 20 ? 2048 : n >= 300000 ? 1024 : n >= 75000 ? 512 : 256;
+	// or five are resident on each), else as many as amortise the region's
+	// flush.  FP64 (whose particles take longest), 1,048,576 of them on 128 x
+	// 128, 200 steps: 2048 per block 73.0 ms, 1024 63.8, 512 60.6; FP32,
+	// 262,144 on 64 x 64, 50 steps: 1024 5.16 ms, 512 4.84, 256 4.99.
+	if(a->f64)
+		a->chunk = n >= 8 << 20 ? 2048 : n >= 4 << 20 ? 1024 : n >= 150000 ? 512 : 256;
+	else
+		a->chunk = n >= 4 << 20 ? 2048 : n >= 1 << 20 ? 1024 : n >= 75000 ? 512 : 256;
 	// tiles of 8 cells, more on sparse and on large grids
 	int tside = 8;
 	while(tside > p->nx || tside > p->ny) tside >>= 1;
