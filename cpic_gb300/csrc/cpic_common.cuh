@@ -17,10 +17,11 @@
 // Every contribution is an integer; integer sums are exact and order
 // independent, so the deposit is deterministic without float atomics.
 // FP64 form: each contribution w*(-q/e0) is rounded to a multiple of
-// 1/qscale and summed per tile in 64-bit shared memory.  Mixed form: the
-// weights w are rounded to multiples of 2^-kWeightBits and summed per tile
-// in 32-bit shared memory (added to global rho and restarted before any
-// sum can wrap, which a check every kCheckChunks chunks detects); the
+// 1/qscale and summed per tile in 64-bit words of shared memory (two 32-bit
+// atomics with a carry).  Mixed form: the weights w are rounded to multiples
+// of 2^-kWeightBits and summed per tile in 32-bit shared memory (added to
+// global rho and restarted before any sum can wrap, which a check every
+// check_chunks(P) chunks detects); the
 // species charge multiplies the tile sums at the flush.
 #pragma once
 #include <cstdint>

@@ -11,14 +11,16 @@
 //   F64 : positions and velocities in FP64, exact reference arithmetic
 //         (this header is compiled with --fmad=false for it); E read from
 //         global memory with the reference's index arithmetic, quirks
-//         included; 64-bit fixed-point shared accumulator.
+//         included; 64-bit fixed-point shared accumulator, added to with
+//         32-bit shared atomics that carry; weights and fixed-point values
+//         on the integer pipes (cpic_bits.h), exactly.
 //   Mix : int32 cell + FP32 offset, FP32 velocity; E staged per tile in
 //         shared memory; 32-bit integer weight accumulator.
 //
 // Skeleton per block (tile t of species s): the tile's particles -- its main
 // region, then the arrivals the previous step left for it -- are read in
-// chunks of kChunk; after one barrier per chunk (every load of the chunk has
-// landed) each particle is pushed, deposited into the tile's shared
+// chunks of kChunk by bulk copies into two stage buffers, each with a "full"
+// and an "empty" mbarrier; each particle is pushed, deposited into the tile's shared
 // accumulator, and written back: stayers compacted in place at the front of
 // the main region through a shared cursor (a warp reserves its run with one
 // shared atomic), movers appended to their destination tile's arrivals in
@@ -996,8 +998,9 @@ k_push(const __grid_constant__ PushArgs a)
 	// with one particle per thread (small tiles) the main region's last,
 	// partial chunk takes arrivals too: a chunk's latency counts there, and
 	// a chunk of arrivals alone is mostly empty (two species 512 x 512, 16
-	// per cell, FP64: 741 us a step in separate chunks, 690 jointly).  With more particles per tile the two extra
-	// instructions per particle cost more than the chunk.
+	// per cell, FP64: 741 us a step in separate chunks, 690 jointly).  With
+	// more particles per tile the two extra instructions per particle cost
+	// more than the chunk.
 	constexpr bool kMerge = P == 1;
 	const int nfull = kMerge ? nm / kChunk : 0;
 	const int rem = nm - nfull * kChunk;
