@@ -34,7 +34,7 @@ METRIC = "particle-steps/s on 1 GB300: FP32-offset vs FP64 plain at ≤1e-5 rel 
 UNIT = "particle-steps/s"
 B_P = {"mixed": 40.0, "fp64": 64.0}     # algorithmic bytes per particle-step
 B_G = {"mixed": 40.0, "fp64": 48.0}     # algorithmic bytes per grid node per step
-KERNELS_PER_STEP = 7                     # the benchmark workload has one species
+KERNELS_PER_STEP = 6                     # the benchmark workload has one species
 
 WORKLOADS = {
     # name: (grid, particles per cell, v0, vth, amp, description)
@@ -267,8 +267,8 @@ def run_ours(args):
            "ms_breakdown": {"particle_kernel": push_ms, "field_stage": field_ms},
            "roofline": roof, "clocks": clk,
            # per step, either form, one species: k_rows_fwd, k_cols, k_rows_inv,
-           # k_E_*, k_spill, k_push, k_tile_order (and the memsets of rho
-           # and of the spill count, not counted)
+           # k_E_*, k_spill, k_push (and k_tile_order every 8th step, not
+           # counted)
            "gpu_launches": args.steps * KERNELS_PER_STEP}
 
     # ---- FP64 plain form on the same workload and the same window of the
