@@ -178,12 +178,19 @@ struct SpillArgs {
 	Spill spill_in[kMaxSpecies];
 };
 
-// Whether the fused kernel takes all species in one launch: while one
-// species' tiles do not fill the GPU.
+// Whether the fused kernel takes all species in one launch.  Launches one
+// after the other each end with a wave of tiles that leaves SMs idle, and
+// the next cannot start before.  Measured with two species (particle kernel,
+// us per step, a launch each -> one launch): FP64 512 x 512 with 16 per
+// cell 665 -> 647, with 64 2394 -> 2362, 256 x 256 with 32 364 -> 338; mixed,
+// 2 particles per thread, 512 x 512 with 16 102 -> 85, with 64 294 -> 286,
+// 1024 x 1024 with 50 829 -> 816.  Mixed with 1 particle per thread gains only
+// below two waves of tiles (1024 tiles 116 -> 103, 4096 tiles 339 -> 353).
 constexpr int kSMs = 152;
-inline bool species_together(const PushArgs &a, int ntiles, int per_sm)
+inline bool species_together(bool mixed, int nspecies, int ntiles, int ppt, int per_sm)
 {
-	return a.nspecies > 1 && ntiles < per_sm * kSMs;
+	if(nspecies < 2 || ppt > 2) return false;
+	return !(mixed && ppt == 1) || ntiles < 2 * per_sm * kSMs;
 }
 
 // The arguments of species sp moved to index 0 (the fused kernel is

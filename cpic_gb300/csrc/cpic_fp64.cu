@@ -120,7 +120,7 @@ cudaError_t launch_push_f64(const PushArgs &a, int ntiles, size_t smem, int ppt,
 	if(!ppt_supported(ppt)) return cudaErrorInvalidValue;
 	cudaError_t e = push_f64_attrs();
 	if(e != cudaSuccess) return e;
-	if(ppt == 1 && species_together(a, ntiles, per_sm))
+	if(ppt == 1 && species_together(false, a.nspecies, ntiles, ppt, per_sm))
 		return launch_pdl(k_push<F64, F64::min_blocks(1), true, 1, true, true>, dim3(ntiles, a.nspecies),
 				kPushThreads, smem, s, a);
 	for(int sp = 0; sp < a.nspecies; sp++)

@@ -231,7 +231,7 @@ cudaError_t launch_push_mix(const PushArgs &a, int ntiles, size_t smem, int ppt,
 	cudaError_t e = push_mix_attrs();
 	if(e != cudaSuccess) return e;
 	const bool hi = per_sm >= Mix::kHiBlocks;
-	if(hi && ppt <= 2 && species_together(a, ntiles, per_sm))
+	if(hi && species_together(true, a.nspecies, ntiles, ppt, per_sm))
 		return launch_pdl(push_mix_all(a.mix[0].id != nullptr, ppt, a.g.pow2 != 0),
 				dim3(ntiles, a.nspecies), kPushThreads, smem, s, a);
 	for(int sp = 0; sp < a.nspecies; sp++)

@@ -912,9 +912,8 @@ struct Mix {
 // Ids: whether the species' store keeps particle ids (always for F64).
 // P: particles per thread per chunk (a chunk is kPushThreads * P particles).
 // GP2: nx and ny are powers of two (the mixed form wraps cells with a mask).
-// Multi: every species in one launch (blockIdx.y), for layouts whose tiles leave
-// the GPU partly idle: two species of 262,144 particles on 128 x 128 take 22 us
-// one after the other.
+// Multi: every species in one launch (blockIdx.y; species_together): two species
+// of 262,144 particles on 128 x 128 take 22 us one after the other.
 template <class F, int MinBlocks = F::kMinBlocks, bool Ids = true, int P = kPPT, bool GP2 = true,
 	bool Multi = false>
 __global__ void __launch_bounds__(kPushThreads, MinBlocks)
