@@ -28,6 +28,7 @@
 #include <cuda.h>            // CUtensorMap (the type only; no driver library is linked)
 #include <cuda_runtime.h>
 #include "cpic_bits.h"
+#include "cpic_layout.h"
 
 namespace cpic {
 
@@ -213,14 +214,6 @@ inline PushArgs species_args(const PushArgs &a, int sp)
 __device__ __forceinline__ int wrap2(int i, int n)
 {
 	return i & (n - 1);
-}
-
-// Periodic wrap for any extent, i in [-n, 2n).
-__host__ __device__ __forceinline__ int wrapn(int i, int n)
-{
-	if(i < 0) i += n;
-	else if(i >= n) i -= n;
-	return i;
 }
 
 // Periodic wrap for any extent and any i (a loop: one or two compares for

@@ -905,8 +905,9 @@ static bool encode_field_map(cpic_ctx *c)
 			CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Tiles of T x T cells.  T need not divide the grid: the tiles of the last
-// column and row are then partly outside it, where no particle lies.
+// Tiles of T x T cells, T below twice either side (layout::field_node).  T need
+// not divide the grid: the tiles of the last column and row are then partly
+// outside it, where no particle lies.
 static void set_tiles(cpic_ctx *c, int T)
 {
 	Grid &g = c->g;
@@ -917,35 +918,6 @@ static void set_tiles(cpic_ctx *c, int T)
 	bits::div_init((uint32_t) g.ntx, g.ntx_mul, g.ntx_sh);
 	c->ntiles = g.ntx * g.nty;
 	c->emap_ok = c->E32 != nullptr && encode_field_map(c);
-}
-
-// The library's tile size for n particles of one species: the largest of 32,
-// 16, 8 and 4 cells whose tiles keep the SMs busy to the end.  One block takes
-// a tile, an SM holds 5 or 6 of them, and a block alone on an SM works off
-// its particles at a fraction of the SM's rate, so: over two waves of tiles
-// (2048), whatever they hold; about a wave (912) if none takes long (8192
-// particles, FP64 2048: its particles take four times as long); a tile per
-// SM if each is short; or next to nothing per tile, where launch latency is
-// all there is.  Smaller tiles than that only add edges.  Measured (particle
-// kernel, us per step, mixed unless said): 128 x 128 with 128 per cell,
-// 16-cell tiles 113, 8-cell 40, 4-cell 31; 256 x 256 with 32, 16-cell 40,
-// 8-cell 31, 4-cell 38; 512 x 512 with 4, 16-cell 25, 8-cell 31, with 100,
-// 16-cell 241, 8-cell 222; 1024 x 1024 with 25, 32-cell 252, 16-cell 233;
-// 2048 x 2048 with 6, 64-cell 402, 32-cell 254, 16-cell 324; FP64 64 x 64
-// with 64, 8-cell 111, 4-cell 46; FP64 512 x 512 with 16, 16-cell 723,
-// 8-cell 690, 4-cell 824.
-static int auto_tile(const cpic_params_t *p, int64_t n)
-{
-	const bool f64 = p->precision == CPIC_FP64;
-	for(int T = 32; T > 4; T >>= 1)
-	{
-		const int64_t tiles = ((p->nx + T - 1) / T) * ((p->ny + T - 1) / T);
-		const int64_t per = n / tiles;
-		if(tiles >= 2048 || (tiles >= 912 && per <= (f64 ? 2048 : 8192))
-				|| (tiles >= 152 && per <= (f64 ? 512 : 1024)) || per <= 128)
-			return T;
-	}
-	return 4;
 }
 
 static void fill_species_step(cpic_ctx *c, PushArgs &a, int64_t iter)
@@ -1617,7 +1589,8 @@ CPIC_API int cpic_create(const cpic_params_t *p, cpic_ctx_t **out)
 	g.idx = 1.0 / g.dx;
 	g.idy = 1.0 / g.dy;
 	// (chosen again by the particles of the first species)
-	const int T = p->tile_x > 0 ? p->tile_x : auto_tile(p, 0);
+	const int T = p->tile_x > 0 ? p->tile_x
+		: layout::auto_tile(p->nx, p->ny, p->precision == CPIC_FP64, 0);
 	int TY = p->tile_y > 0 ? p->tile_y : T;
 	if(!pow2(T) || !pow2(TY) || (p->tile_x > 0 && (p->nx % T || p->ny % TY)) || T != TY)
 	{
@@ -1866,7 +1839,7 @@ CPIC_API int cpic_add_species(cpic_ctx_t *c, double q, double m, int64_t n,
 
 	int s = c->nspecies;
 	if(s == 0 && n > 0 && c->p.tile_x <= 0)
-		set_tiles(c, auto_tile(&c->p, n));
+		set_tiles(c, layout::auto_tile(c->p.nx, c->p.ny, c->precision == CPIC_FP64, n));
 	SpeciesHost &S = c->sp[s];
 	memset((void *) &S, 0, sizeof(S));
 	S.q = q; S.m = m; S.n = n;

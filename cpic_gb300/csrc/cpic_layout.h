@@ -1,0 +1,64 @@
+// cpic_layout.h -- the tile layout's host rules and the index arithmetic that
+// depends on them.  Plain C++ (host and device), so a CPU test checks the
+// rules' results over the whole range of grids against the ranges that the
+// kernels' indices need.
+#pragma once
+#include <cstdint>
+
+#include "cpic_bits.h"
+
+namespace cpic {
+
+// Periodic wrap for any extent, i in [-n, 2n).
+CPIC_HD int wrapn(int i, int n)
+{
+	if(i < 0) i += n;
+	else if(i >= n) i -= n;
+	return i;
+}
+
+namespace layout {
+
+// Along one side of n nodes: the node held at place l (0 .. T) of the field
+// tile whose first node is t0 (a multiple of the tile size T, below n).  T < 2n
+// keeps t0 + l below 2n: with one tile t0 is 0, with more T is below n.
+CPIC_HD int field_node(int t0, int l, int n)
+{
+	return wrapn(t0 + l, n);
+}
+
+// The library's tile size for n particles of one species: the largest of 32,
+// 16, 8 and 4 cells whose tiles keep the SMs busy to the end.  One block takes
+// a tile, an SM holds 5 or 6 of them, and a block alone on an SM works off
+// its particles at a fraction of the SM's rate, so: over two waves of tiles
+// (2048), whatever they hold; about a wave (912) if none takes long (8192
+// particles, FP64 2048: its particles take four times as long); a tile per
+// SM if each is short; or next to nothing per tile, where launch latency is
+// all there is.  Smaller tiles than that only add edges.  Measured (particle
+// kernel, us per step, mixed unless said): 128 x 128 with 128 per cell,
+// 16-cell tiles 113, 8-cell 40, 4-cell 31; 256 x 256 with 32, 16-cell 40,
+// 8-cell 31, 4-cell 38; 512 x 512 with 4, 16-cell 25, 8-cell 31, with 100,
+// 16-cell 241, 8-cell 222; 1024 x 1024 with 25, 32-cell 252, 16-cell 233;
+// 2048 x 2048 with 6, 64-cell 402, 32-cell 254, 16-cell 324; FP64 64 x 64
+// with 64, 8-cell 111, 4-cell 46; FP64 512 x 512 with 16, 16-cell 723,
+// 8-cell 690, 4-cell 824.
+//
+// A tile below twice the shorter side at most (field_node): its first power of
+// two that covers that side, beyond which a tile only holds places of no cell.
+inline int auto_tile(int64_t nx, int64_t ny, bool f64, int64_t n)
+{
+	int T = 32;
+	while(T >= 2 * nx || T >= 2 * ny) T >>= 1;
+	for(; T > 4; T >>= 1)
+	{
+		const int64_t tiles = ((nx + T - 1) / T) * ((ny + T - 1) / T);
+		const int64_t per = n / tiles;
+		if(tiles >= 2048 || (tiles >= 912 && per <= (f64 ? 2048 : 8192))
+				|| (tiles >= 152 && per <= (f64 ? 512 : 1024)) || per <= 128)
+			return T;
+	}
+	return 4;
+}
+
+} // namespace layout
+} // namespace cpic

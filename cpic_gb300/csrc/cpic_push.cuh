@@ -831,7 +831,7 @@ struct Mix {
 		for(int i = threadIdx.x; i < WE * (g.ty + 1); i += blockDim.x)
 		{
 			int lx = i % WE, ly = i / WE;
-			int gx = wrapn(tx0 + lx, g.nx), gy = wrapn(ty0 + ly, g.ny);
+			int gx = layout::field_node(tx0, lx, g.nx), gy = layout::field_node(ty0, ly, g.ny);
 			Et[ly * (g.tx + 2) + lx] = a.E32[(int64_t) gy * g.nx + gx];
 		}
 		return Et;
