@@ -373,11 +373,14 @@ __device__ __forceinline__ void pdl_wait()
 
 // Lets the next kernel's blocks start, and run what touches no data of the
 // chain, once every block of this one has got here; without it they start
-// when this one's blocks are done.  Only in kernels that leave the SMs
-// nearly empty (the spill pass, the tile order): next to a working kernel the
-// early blocks go where there is room, not where they will run best, and
+// when this one's blocks are done.  Only in a kernel that leaves the SMs
+// nearly empty (the tile order, a block per species): next to a working kernel
+// the early blocks go where there is room, not where they will run best, and
 // stay there (a 512 x 512 FP64 solve, one or two blocks per SM and kernel: 99
 // us with triggers everywhere, 58 without; 250 x 150 FP64 step 168 and 140).
+// The spill pass is such a working kernel when it has records: with a trigger
+// there, the particle kernel's blocks shared the SMs unevenly, and those that
+// ran late found the spill list taken by the others.
 __device__ __forceinline__ void pdl_trigger()
 {
 	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -1231,7 +1231,7 @@ k_spill(const SpillArgs sa)
 {
 	const PushArgs &a = sa.p;
 	const Grid &g = a.g;
-	pdl_trigger();
+	// (no trigger: with records to push this is a working kernel)
 	pdl_wait();
 	for(int s = 0; s < a.nspecies; s++)
 	{
