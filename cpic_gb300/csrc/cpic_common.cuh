@@ -33,34 +33,6 @@
 namespace cpic {
 
 constexpr int kMaxSpecies = 8;
-// Block shape of the fused particle kernel (build-time knobs).
-#ifndef CPIC_PUSH_THREADS
-#define CPIC_PUSH_THREADS 256
-#endif
-#ifndef CPIC_PPT
-#define CPIC_PPT 2
-#endif
-constexpr int kPushThreads = CPIC_PUSH_THREADS;
-// Particles per thread per chunk: the default, and the compiled instances of
-// the fused kernel a context may choose from (the autotuner times them).
-constexpr int kPPT = CPIC_PPT;
-constexpr int kPPTChoices[] = {1, 2, 4};
-constexpr int kWeightBits = 18;
-// Particles per chunk with P particles per thread.
-__host__ __device__ constexpr int chunk_of(int P) { return kPushThreads * P; }
-// 32-bit (unsigned) shared weight sums: a node gains at most 2^kWeightBits
-// per particle, so check_chunks(P) chunks add at most 2^32 - 2^kCheckBits to
-// any node; a check every check_chunks(P) chunks that finds every node below
-// 2^kCheckBits keeps every sum below 2^32 until the next check.  A check
-// costs a block barrier and a pass over the sums: every 31 chunks instead of
-// every 8 (with a limit of 2^30 at the checks and 2^31 between them) took
-// 1.4 % off the fused kernel on the two-stream 2048x2048 benchmark.
-constexpr int kCheckBits = 27;
-__host__ __device__ constexpr int check_chunks(int P)
-{
-	return (int) (((1ll << 32) - (1ll << kCheckBits)) / ((long long) chunk_of(P) << kWeightBits));
-}
-static_assert(check_chunks(4) >= 1, "chunk too large for 32-bit weight sums");
 inline bool ppt_supported(int P) { return P == 1 || P == 2 || P == 4; }
 
 // Device status bits (sticky until the host clears them).

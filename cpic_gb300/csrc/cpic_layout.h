@@ -9,6 +9,40 @@
 
 namespace cpic {
 
+// Block shape of the fused particle kernel (build-time knobs).
+#ifndef CPIC_PUSH_THREADS
+#define CPIC_PUSH_THREADS 256
+#endif
+#ifndef CPIC_PPT
+#define CPIC_PPT 2
+#endif
+constexpr int kPushThreads = CPIC_PUSH_THREADS;
+// Particles per thread per chunk: the default, and the compiled instances of
+// the fused kernel a context may choose from (the autotuner times them).
+constexpr int kPPT = CPIC_PPT;
+constexpr int kPPTChoices[] = {1, 2, 4};
+constexpr int kWeightBits = 18;
+// Particles per chunk with P particles per thread.
+CPIC_HD constexpr int chunk_of(int P) { return kPushThreads * P; }
+// 32-bit (unsigned) shared weight sums: a node gains at most 2^kWeightBits
+// per particle.  A check every check_chunks(P) chunks folds the sums into the
+// grid when it sees a node at 2^kCheckBits or above.  It reads the sums before
+// its barrier, when other warps may still owe deposits of the chunks before:
+// a chunk is issued once every warp has released the one that was in its
+// buffer, which a warp does before the last push, so a warp can be two chunks
+// and one push behind another.  A node that the check passes is therefore
+// below 2^kCheckBits plus those deposits, and the interval leaves room for
+// them: every sum stays below 2^32.  A check costs a block barrier and a pass
+// over the sums (two-stream 2048 x 2048 benchmark: every 8 chunks, with a limit
+// of 2^30, took 1.4 % longer over the whole kernel than every 31).
+constexpr int kCheckBits = 27;
+CPIC_HD constexpr int owed_deposits(int P) { return 2 * chunk_of(P) + kPushThreads; }
+CPIC_HD constexpr int check_chunks(int P)
+{
+	return (int) (((((1ll << 32) - (1ll << kCheckBits)) >> kWeightBits) - owed_deposits(P)) / chunk_of(P));
+}
+static_assert(check_chunks(4) >= 1, "chunk too large for 32-bit weight sums");
+
 // Periodic wrap for any extent, i in [-n, 2n).
 CPIC_HD int wrapn(int i, int n)
 {

@@ -1052,10 +1052,12 @@ k_push(const __grid_constant__ PushArgs a)
 		const int clen = ck.n + ck.na;
 		if(ci > 0 && ci % kCheckChunks == 0)
 		{
-			// every deposit of the previous chunks precedes the check (and
-			// the fold), and the fold precedes every later deposit.  At
-			// typical densities a node's sum over the whole tile stays far
-			// below 2^kCheckBits and the fold never runs.
+			// the sums are read before the barrier: this warp's deposits are
+			// in, others may be owed (check_chunks leaves room for them).
+			// Every deposit of the previous chunks precedes the fold, and the
+			// fold precedes every later one.  At typical densities a node's
+			// sum over the whole tile stays far below 2^kCheckBits and the
+			// fold never runs.
 			if(__syncthreads_or(F::near_full(fsm, W, g.tx)))
 			{
 				F::fold(a, s, fsm, W, H, tx0, ty0);
