@@ -2638,7 +2638,14 @@ CPIC_API int cpic_ensemble_run(cpic_ensemble_t *e, int64_t nsteps, double *ms_gr
 		for(int64_t k = 0; k < pairs; k++)
 		{
 			CK(cudaGraphLaunch(e->exec, e->origin));
-			for(cpic_ctx *c : e->runs) c->iter += 2;
+			for(cpic_ctx *c : e->runs)
+			{
+				c->iter += 2;
+				// what the host knew of the spill lists and of the other
+				// charge buffer is from before the replay
+				c->spill_empty = false;
+				c->next_clean = false;
+			}
 			if((k & 1) == 1 || k + 1 == pairs)
 			{
 				CK(cudaEventRecord(e->t1, e->origin));
