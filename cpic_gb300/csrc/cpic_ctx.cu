@@ -45,6 +45,8 @@ struct SpeciesHost {
 	Tiles tiles;
 	Spill spill[2];          // ping-pong: spill[cur] is the input
 	double vmax;              // largest initial |u| component
+	double move;              // mean |dx| + |dy| per step in cells: when loaded,
+	                          // more when a later re-layout finds more
 	double wq_mult;           // mixed form: fixed-point units per weight unit
 };
 
@@ -104,7 +106,7 @@ struct cpic_ctx {
 	double *part_h;           // pinned: partial sums of the field energy (2 ny)
 	CUtensorMap emap;         // mixed form: E32 as 2D tiles for the fused kernel
 	bool emap_ok;
-	unsigned long long *counter_pair;  // two device scalars (upload check)
+	unsigned long long *upload_chk;    // kUploadChk device scalars (k_upload_check)
 };
 
 constexpr int kCtl = 1 + 2 * kMaxSpecies;
@@ -332,6 +334,56 @@ __global__ void k_rb_copy(const PushArgs olda, const PushArgs newa, int s)
 		typename F::Rec r = F::load(olda, s, i < n ? ob + i : oab + (i - n));
 		F::store(newa, s, nb + i, r);
 	}
+}
+
+// |dx| + |dy| of a step in whole kMoveUnits-ths of a cell, kMoveMax cells at
+// most (also for a speed beyond FP32).  cx, cy: cells per step and unit of
+// velocity.  Integers, so that their sums are the same in any order.
+constexpr float kMoveUnits = 256.0f, kMoveMax = 32768.0f;
+__device__ __forceinline__ unsigned move_units(float u, float v, float cx, float cy)
+{
+	return (unsigned) (kMoveUnits * fminf(fabsf(u) * cx + fabsf(v) * cy, kMoveMax));
+}
+
+// The sum of move_units over a species' particles (out[0]) and their number
+// (out[1]), of every fourth run of 256 in each tile's main region and arrivals.
+template <class F>
+__global__ void k_move_tiles(const PushArgs a, int s, float cx, float cy, unsigned long long *out)
+{
+	const int t = blockIdx.x;
+	const Tiles &T = a.tiles[s];
+	const int n = T.cnt[t], na = min(T.acnt[a.arr_r][t], T.acap[t]);
+	const int64_t b = T.base[t], ab = T.abase[t] + (a.arr_r ? T.abuf1 : 0);
+	unsigned long long sum = 0, num = 0;
+	for(int i = threadIdx.x; i < n + na; i += 4 * blockDim.x)
+	{
+		const typename F::Rec r = F::load(a, s, i < n ? b + i : ab + (i - n));
+		sum += move_units((float) r.ux, (float) r.uy, cx, cy);
+		num++;
+	}
+	for(int o = 16; o > 0; o >>= 1)
+	{
+		sum += __shfl_xor_sync(0xffffffffu, sum, o);
+		num += __shfl_xor_sync(0xffffffffu, num, o);
+	}
+	if((threadIdx.x & 31) == 0 && num)
+	{
+		atomicAdd(&out[0], sum);
+		atomicAdd(&out[1], num);
+	}
+}
+
+// The same over staged records, all of them.
+__global__ void k_move_list(int64_t n, const Spill S, float cx, float cy, unsigned long long *out)
+{
+	unsigned long long sum = 0;
+	for(int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n;
+			i += (int64_t) gridDim.x * blockDim.x)
+		sum += move_units((float) S.ux[i], (float) S.uy[i], cx, cy);
+	for(int o = 16; o > 0; o >>= 1)
+		sum += __shfl_xor_sync(0xffffffffu, sum, o);
+	if((threadIdx.x & 31) == 0 && sum) atomicAdd(&out[0], sum);
+	if(blockIdx.x == 0 && threadIdx.x == 0) out[1] = (unsigned long long) n;
 }
 
 // Particles of each tile: its main region's and its pending arrivals.
@@ -624,10 +676,13 @@ __global__ void k_rb_cursors(int nt, const int64_t *base, const int32_t *neg,
 
 // Upload check, numbering and Y wrap of a staged species.  out[0]: any
 // invalid record (x outside [0, Lx], non-finite y, ux, uy); out[1]: the
-// largest |ux|, |uy| as the bit pattern of a non-negative double.
-__global__ void k_upload_check(int64_t n, Spill S, double Lx, double Ly, unsigned long long *out)
+// largest |ux|, |uy| as the bit pattern of a non-negative double; out[2]: the
+// sum of move_units.
+constexpr int kUploadChk = 3;
+__global__ void k_upload_check(int64_t n, Spill S, double Lx, double Ly, float cx, float cy,
+		unsigned long long *out)
 {
-	unsigned long long bad = 0;
+	unsigned long long bad = 0, move = 0;
 	double vm = 0.0;
 	for(int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n;
 			i += (int64_t) gridDim.x * blockDim.x)
@@ -638,6 +693,7 @@ __global__ void k_upload_check(int64_t n, Spill S, double Lx, double Ly, unsigne
 		else
 		{
 			vm = fmax(vm, fmax(fabs(u), fabs(v)));
+			move += move_units((float) u, (float) v, cx, cy);
 			// one periodic wrap in Y, as the initial global exchange does
 			// (sim_pre_step -> comm_plasma(sim, 1), comm_plasma.c:1087-1112)
 			if(y >= Ly) S.y[i] = y - Ly;
@@ -649,10 +705,12 @@ __global__ void k_upload_check(int64_t n, Spill S, double Lx, double Ly, unsigne
 	{
 		bad |= __shfl_xor_sync(0xffffffffu, bad, o);
 		vm = fmax(vm, __shfl_xor_sync(0xffffffffu, vm, o));
+		move += __shfl_xor_sync(0xffffffffu, move, o);
 	}
 	if((threadIdx.x & 31) == 0)
 	{
 		if(bad) atomicOr(&out[0], 1ULL);
+		if(move) atomicAdd(&out[2], move);
 		atomicMax(&out[1], (unsigned long long) __double_as_longlong(vm));
 	}
 }
@@ -1083,6 +1141,10 @@ static void launch_rb_count(const Grid &g, const Spill &S, int64_t cnt, int32_t 
 		k_rb_count<F><<<grid_blocks(cnt), 256, 0, st>>>(g, S, cnt, newcnt);
 }
 
+// move_units' factors
+static float move_cx(const cpic_ctx *c) { return (float) (c->p.dt * c->g.idx); }
+static float move_cy(const cpic_ctx *c) { return (float) (c->p.dt * c->g.idy); }
+
 // Largest tile count of the block-local upload sort (its scatter keeps
 // 4 ints per tile in shared memory: 128 KB).
 constexpr int kBlkSortMaxTiles = 8192;
@@ -1090,7 +1152,8 @@ constexpr int kBlkSortMaxTiles = 8192;
 // Counting-sort rebuild of species s: its tiles (unless `fresh`), its
 // current spill input and an optional staging list are merged into a new
 // layout whose tile capacities follow the new counts.
-static int rebuild_species(cpic_ctx *c, int s, bool fresh, const Spill *staging, int64_t nstage)
+static int rebuild_species(cpic_ctx *c, int s, bool fresh, const Spill *staging, int64_t nstage,
+		bool measure = true)
 {
 	SpeciesHost &S = c->sp[s];
 	int nt = c->ntiles;
@@ -1101,6 +1164,22 @@ static int rebuild_species(cpic_ctx *c, int s, bool fresh, const Spill *staging,
 	CK(cudaStreamSynchronize(st));
 	if(nspill > spin.capacity) nspill = spin.capacity;
 
+	// how far the particles move now (cpic_add_species has measured it)
+	unsigned long long hmove[2] = {0, 0};
+	if(measure)
+	{
+		const PushArgs a = make_args(c, c->spill_cur);
+		CK(cudaMemsetAsync(c->upload_chk, 0, sizeof(hmove), st));
+		if(fresh)
+			k_move_list<<<grid_blocks(nstage), 256, 0, st>>>(nstage, *staging, move_cx(c), move_cy(c),
+					c->upload_chk);
+		else if(c->precision == CPIC_MIXED)
+			k_move_tiles<Mix><<<nt, 256, 0, st>>>(a, s, move_cx(c), move_cy(c), c->upload_chk);
+		else
+			k_move_tiles<F64><<<nt, 256, 0, st>>>(a, s, move_cx(c), move_cy(c), c->upload_chk);
+		CK(cudaGetLastError());
+		CK(cudaMemcpyAsync(hmove, c->upload_chk, sizeof(hmove), cudaMemcpyDeviceToHost, st));
+	}
 	int32_t *newcnt = nullptr, *fill = nullptr, *negcnt = nullptr;
 	CK(cudaMalloc(&newcnt, nt * sizeof(int32_t)));
 	CK(cudaMalloc(&fill, nt * sizeof(int32_t)));
@@ -1153,6 +1232,8 @@ static int rebuild_species(cpic_ctx *c, int s, bool fresh, const Spill *staging,
 	std::vector<int32_t> hc(nt);
 	CK(cudaMemcpyAsync(hc.data(), newcnt, nt * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
 	CK(cudaStreamSynchronize(st));
+	if(hmove[1] > 0)
+		S.move = std::max(S.move, (double) hmove[0] / kMoveUnits / (double) hmove[1]);
 
 	// capacities: slack_pct % slack (25 % at first, doubled after every
 	// rebuild forced by an overflow, up to 200 %) plus 64 slots, rounded
@@ -1162,16 +1243,19 @@ static int rebuild_species(cpic_ctx *c, int s, bool fresh, const Spill *staging,
 	// the particles of the two-stream workload between tiles), more as
 	// overflows raise the slack (a quarter of it in each buffer, so that a
 	// store at 200 % slack holds 4x its particles: two such stores, the
-	// current one and the alternate, of both forms fit in HBM at 2048^2)
+	// current one and the alternate, of both forms fit in HBM at 2048^2),
+	// and more for a species whose speed takes more than that over a tile's
+	// edge in a step (layout::arrivals_pct)
 	std::vector<int64_t> hb(nt), hab(nt);
 	std::vector<int32_t> hcap(nt), hacap(nt);
 	int64_t total = 0, atotal = 0, n = 0;
-	const int arr_pct = std::max(25, c->slack_pct / 4);
+	const int arr_pct = layout::arrivals_pct(S.move, c->g.tx, c->slack_pct);
 	for(int t = 0; t < nt; t++)
 	{
-		int64_t cap = hc[t] + hc[t] * c->slack_pct / 100 + 64;
+		const int64_t count = hc[t];
+		int64_t cap = count + count * c->slack_pct / 100 + 64;
 		cap = (cap + 31) & ~(int64_t) 31;
-		int64_t acap = hc[t] * arr_pct / 100 + 64;
+		int64_t acap = count * arr_pct / 100 + 64;
 		acap = (acap + 31) & ~(int64_t) 31;
 		if(cap > INT32_MAX || acap > INT32_MAX) return CPIC_ECAPACITY;
 		hb[t] = total;
@@ -1632,7 +1716,7 @@ CPIC_API int cpic_create(const cpic_params_t *p, cpic_ctx_t **out)
 	AL(c->cosy, g.ny * sizeof(double));
 	AL(c->mean, sizeof(double));
 	AL(c->counter, sizeof(int32_t));
-	AL(c->counter_pair, 2 * sizeof(unsigned long long));
+	AL(c->upload_chk, kUploadChk * sizeof(unsigned long long));
 	if(c->precision == CPIC_FP64)
 	{
 		AL(c->phi64, ng * sizeof(double));
@@ -1739,7 +1823,7 @@ CPIC_API void cpic_destroy(cpic_ctx_t *c)
 	cudaFree(c->phi32); cudaFree(c->E32); cudaFree(c->spec64); cudaFree(c->spec32);
 	cudaFree(c->twx64); cudaFree(c->twy64); cudaFree(c->twx32); cudaFree(c->twy32);
 	cudaFree(c->cosx); cudaFree(c->cosy); cudaFree(c->green64); cudaFree(c->green32); cudaFree(c->mean);
-	cudaFree(c->ctl); cudaFree(c->scratch); cudaFree(c->counter); cudaFree(c->counter_pair);
+	cudaFree(c->ctl); cudaFree(c->scratch); cudaFree(c->counter); cudaFree(c->upload_chk);
 	if(c->stream) cudaStreamDestroy(c->stream);
 	if(c->part_h) cudaFreeHost(c->part_h);
 	delete c;
@@ -1816,18 +1900,18 @@ CPIC_API int cpic_add_species(cpic_ctx_t *c, double q, double m, int64_t n,
 	Spill stg;
 	memset(&stg, 0, sizeof(stg));
 	if((r = alloc_spill(stg, (int32_t) std::max<int64_t>(n, 1), st))) return r;
-	double vmax = 0.0;
+	double vmax = 0.0, move = 0.0;
 	if(n > 0)
 	{
 		CK(cudaMemcpyAsync(stg.x, x, n * sizeof(double), cudaMemcpyHostToDevice, st));
 		CK(cudaMemcpyAsync(stg.y, y, n * sizeof(double), cudaMemcpyHostToDevice, st));
 		CK(cudaMemcpyAsync(stg.ux, ux, n * sizeof(double), cudaMemcpyHostToDevice, st));
 		CK(cudaMemcpyAsync(stg.uy, uy, n * sizeof(double), cudaMemcpyHostToDevice, st));
-		unsigned long long *chk = reinterpret_cast<unsigned long long *>(c->counter_pair);
-		CK(cudaMemsetAsync(chk, 0, 2 * sizeof(unsigned long long), st));
-		k_upload_check<<<grid_blocks(n, 256, 8 * 152), 256, 0, st>>>(n, stg, c->p.Lx, c->p.Ly, chk);
-		unsigned long long h[2];
-		CK(cudaMemcpyAsync(h, chk, sizeof(h), cudaMemcpyDeviceToHost, st));
+		unsigned long long h[kUploadChk];
+		CK(cudaMemsetAsync(c->upload_chk, 0, sizeof(h), st));
+		k_upload_check<<<grid_blocks(n, 256, 8 * 152), 256, 0, st>>>(n, stg, c->p.Lx, c->p.Ly,
+				move_cx(c), move_cy(c), c->upload_chk);
+		CK(cudaMemcpyAsync(h, c->upload_chk, sizeof(h), cudaMemcpyDeviceToHost, st));
 		CK(cudaStreamSynchronize(st));
 		if(h[0])
 		{
@@ -1835,6 +1919,7 @@ CPIC_API int cpic_add_species(cpic_ctx_t *c, double q, double m, int64_t n,
 			return CPIC_EINVAL;
 		}
 		memcpy(&vmax, &h[1], sizeof(double));
+		move = (double) h[2] / kMoveUnits / (double) n;
 	}
 
 	int s = c->nspecies;
@@ -1844,6 +1929,7 @@ CPIC_API int cpic_add_species(cpic_ctx_t *c, double q, double m, int64_t n,
 	memset((void *) &S, 0, sizeof(S));
 	S.q = q; S.m = m; S.n = n;
 	S.vmax = vmax;
+	S.move = move;
 	// the fused kernel's instance when the caller left it to the library.
 	// FP64: 1 particle per thread; the kernel's arithmetic is long enough to
 	// hide a chunk's latency, and a second copy of its code misses the
@@ -1884,7 +1970,7 @@ CPIC_API int cpic_add_species(cpic_ctx_t *c, double q, double m, int64_t n,
 
 	// counting sort of the staged particles into the tiles
 	update_qscale(c);
-	r = rebuild_species(c, s, true, &stg, n);
+	r = rebuild_species(c, s, true, &stg, n, false);
 	free_spill(stg);
 	if(r) return r;
 	// halo: a particle displaced by at most D cells in a step deposits

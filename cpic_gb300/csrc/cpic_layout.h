@@ -3,6 +3,7 @@
 // rules' results over the whole range of grids against the ranges that the
 // kernels' indices need.
 #pragma once
+#include <algorithm>
 #include <cstdint>
 
 #include "cpic_bits.h"
@@ -92,6 +93,21 @@ inline int auto_tile(int64_t nx, int64_t ny, bool f64, int64_t n)
 			return T;
 	}
 	return 4;
+}
+
+// Room for arrivals in percent of a tile's particles, for a species that moves
+// `move` cells per step on average (|dx| + |dy|): at most move / T of the
+// particles leave their tile of T cells in a step, and as many come in where
+// the density is even; a tenth more than that.  At least a quarter, or a
+// quarter of the slack that overflows have raised.  Without room for them most
+// movers go through the spill list, which holds an eighth of a species (64 x
+// 64, 64 per cell, two beams of 2.5 cells per step in 4-cell tiles: the list
+// is full in the second step, and tiles overflow before the next check).
+inline int arrivals_pct(double move, int T, int slack_pct)
+{
+	const double leave = move < T ? move / T : 1.0;
+	const int pct = (int) (110.0 * leave) + 1;
+	return std::max(std::max(25, slack_pct / 4), pct);
 }
 
 } // namespace layout

@@ -45,8 +45,26 @@ static void check_grid(int nx, int ny)
 		}
 }
 
+// Room for the movers of a plasma at any speed, never less than a quarter or
+// a quarter of the slack.
+static void check_arrivals()
+{
+	for(int T = 1; T <= 64; T *= 2)
+		for(int slack : {0, 25, 50, 100, 200, 1000})
+			for(double move : {0.0, 1e-300, 0.01, 0.3, 1.0, 2.5, 3.999, 4.0, 12.0, 63.9, 64.1, 32768.0})
+			{
+				const int pct = layout::arrivals_pct(move, T, slack);
+				const double leave = std::min(1.0, move / T);
+				if(pct >= 25 && pct >= slack / 4 && pct >= 109.99 * leave && pct <= std::max(111, slack / 4))
+					continue;
+				bad++;
+				std::printf("room for arrivals: %d %% at %g cells per step, T %d, slack %d\n", pct, move, T, slack);
+			}
+}
+
 int main()
 {
+	check_arrivals();
 	std::vector<int> sides;
 	for(int n = 4; n <= 70; n++) sides.push_back(n);
 	for(int n = 128; n <= 16384; n *= 2)
