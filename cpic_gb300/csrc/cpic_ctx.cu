@@ -386,6 +386,25 @@ __global__ void k_move_list(int64_t n, const Spill S, float cx, float cy, unsign
 	if(blockIdx.x == 0 && threadIdx.x == 0) out[1] = (unsigned long long) n;
 }
 
+// Every particle of a species' main regions into a list.
+template <class F>
+__global__ void k_list_tiles(const PushArgs a, int s, Spill out)
+{
+	__shared__ int first;
+	const int t = blockIdx.x;
+	const int n = a.tiles[s].cnt[t];
+	const int64_t b = a.tiles[s].base[t];
+	if(threadIdx.x == 0) first = atomicAdd(out.count, n);
+	__syncthreads();
+	for(int i = threadIdx.x; i < n && first + i < out.capacity; i += blockDim.x)
+	{
+		const typename F::Rec r = F::load(a, s, b + i);
+		const int k = first + i;
+		F::to_spill_rec(r, a.g, out.x[k], out.y[k], out.ux[k], out.uy[k]);
+		out.id[k] = r.id;
+	}
+}
+
 // Particles of each tile: its main region's and its pending arrivals.
 __global__ void k_tile_total(int nt, const Tiles T, int abuf, int32_t *out)
 {
@@ -1119,6 +1138,33 @@ static void free_spill(Spill &S, bool own_count = true)
 	memset(&S, 0, sizeof(S));
 }
 
+// A species' tile arrays, empty tiles in index order.
+static int alloc_tiles(Tiles &T, int nt, cudaStream_t st)
+{
+	CK(cudaMalloc(&T.base, nt * sizeof(int64_t)));
+	CK(cudaMalloc(&T.cap, nt * sizeof(int32_t)));
+	CK(cudaMalloc(&T.cnt, nt * sizeof(int32_t)));
+	CK(cudaMalloc(&T.abase, nt * sizeof(int64_t)));
+	CK(cudaMalloc(&T.acap, nt * sizeof(int32_t)));
+	CK(cudaMalloc(&T.acnt[0], nt * sizeof(int32_t)));
+	CK(cudaMalloc(&T.acnt[1], nt * sizeof(int32_t)));
+	CK(cudaMalloc(&T.order, nt * sizeof(int32_t)));
+	k_iota<<<grid_blocks(nt), 256, 0, st>>>(nt, T.order);
+	CK(cudaGetLastError());
+	CK(cudaMemsetAsync(T.cnt, 0, nt * sizeof(int32_t), st));
+	CK(cudaMemsetAsync(T.acnt[0], 0, nt * sizeof(int32_t), st));
+	CK(cudaMemsetAsync(T.acnt[1], 0, nt * sizeof(int32_t), st));
+	return CPIC_OK;
+}
+
+static void free_tiles(Tiles &T)
+{
+	cudaFree(T.base); cudaFree(T.cap); cudaFree(T.cnt);
+	cudaFree(T.abase); cudaFree(T.acap);
+	cudaFree(T.acnt[0]); cudaFree(T.acnt[1]); cudaFree(T.order);
+	memset(&T, 0, sizeof(T));
+}
+
 template <class F>
 static void launch_rb_copy(const PushArgs &o, const PushArgs &n, int s, int nt, cudaStream_t st)
 {
@@ -1593,6 +1639,54 @@ static int normalize(cpic_ctx *c)
 	return CPIC_OK;
 }
 
+// The species loaded so far in tiles of T cells instead of the present ones.
+static int change_tiles(cpic_ctx *c, int T)
+{
+	const int ns = c->nspecies, cu = c->precision == CPIC_MIXED ? 1 : 0;
+	cudaStream_t st = c->stream;
+	if(ns == 0)
+	{
+		set_tiles(c, T);
+		return CPIC_OK;
+	}
+	int r = normalize(c);
+	if(r) return r;
+	// all particles out, then all in: a list's records are exact
+	// (to_spill_rec); what can fail for want of memory comes before the change
+	const int nt = (int) (((int64_t) (c->g.nx + T - 1) / T) * ((c->g.ny + T - 1) / T));
+	Spill list[kMaxSpecies];
+	Tiles tiles[kMaxSpecies];
+	memset(list, 0, sizeof(list));
+	memset(tiles, 0, sizeof(tiles));
+	const PushArgs a = make_args(c, c->spill_cur);
+	for(int s = 0; s < ns && r == CPIC_OK; s++)
+	{
+		r = alloc_spill(list[s], (int32_t) std::max<int64_t>(c->sp[s].n, 1), st, cu);
+		if(r == CPIC_OK) r = alloc_tiles(tiles[s], nt, st);
+		if(r) break;
+		if(cu) k_list_tiles<Mix><<<c->ntiles, 256, 0, st>>>(a, s, list[s]);
+		else k_list_tiles<F64><<<c->ntiles, 256, 0, st>>>(a, s, list[s]);
+		if(cudaGetLastError() != cudaSuccess) r = CPIC_ECUDA;
+	}
+	if(cudaStreamSynchronize(st) != cudaSuccess && r == CPIC_OK) r = CPIC_ECUDA;
+	if(r == CPIC_OK)
+	{
+		set_tiles(c, T);
+		c->order_mode = 0;
+		c->push_per_sm = 0;
+		for(int s = 0; s < ns; s++)
+			std::swap(c->sp[s].tiles, tiles[s]);
+		for(int s = 0; s < ns && r == CPIC_OK; s++)
+			r = rebuild_species(c, s, true, &list[s], c->sp[s].n, false);
+	}
+	for(int s = 0; s < ns; s++)
+	{
+		free_spill(list[s]);
+		free_tiles(tiles[s]);
+	}
+	return r;
+}
+
 static int field_stage_async(cpic_ctx *c)
 {
 	cudaStream_t st = c->stream;
@@ -1672,7 +1766,7 @@ CPIC_API int cpic_create(const cpic_params_t *p, cpic_ctx_t **out)
 	// interpolate_f2p_E / interpolate_p2f_rho, interpolate.c:303-304
 	g.idx = 1.0 / g.dx;
 	g.idy = 1.0 / g.dy;
-	// (chosen again by the particles of the first species)
+	// (chosen again as species are added)
 	const int T = p->tile_x > 0 ? p->tile_x
 		: layout::auto_tile(p->nx, p->ny, p->precision == CPIC_FP64, 0);
 	int TY = p->tile_y > 0 ? p->tile_y : T;
@@ -1812,9 +1906,7 @@ CPIC_API void cpic_destroy(cpic_ctx_t *c)
 		SpeciesHost &S = c->sp[s];
 		free_store(c, S, false);
 		free_store(c, S, true);
-		cudaFree(S.tiles.base); cudaFree(S.tiles.cap); cudaFree(S.tiles.cnt);
-		cudaFree(S.tiles.abase); cudaFree(S.tiles.acap);
-		cudaFree(S.tiles.acnt[0]); cudaFree(S.tiles.acnt[1]); cudaFree(S.tiles.order);
+		free_tiles(S.tiles);
 		free_spill(S.spill[0], false);
 		free_spill(S.spill[1], false);
 	}
@@ -1922,9 +2014,20 @@ CPIC_API int cpic_add_species(cpic_ctx_t *c, double q, double m, int64_t n,
 		move = (double) h[2] / kMoveUnits / (double) n;
 	}
 
+	// the library's tiles follow the largest species, whatever the order in
+	// which they are added
 	int s = c->nspecies;
-	if(s == 0 && n > 0 && c->p.tile_x <= 0)
-		set_tiles(c, layout::auto_tile(c->p.nx, c->p.ny, c->precision == CPIC_FP64, n));
+	if(c->p.tile_x <= 0)
+	{
+		int64_t most = n;
+		for(int k = 0; k < s; k++) most = std::max(most, c->sp[k].n);
+		const int T = layout::auto_tile(c->p.nx, c->p.ny, c->precision == CPIC_FP64, most);
+		if(T != c->g.tx && (r = change_tiles(c, T)))
+		{
+			free_spill(stg);
+			return r;
+		}
+	}
 	SpeciesHost &S = c->sp[s];
 	memset((void *) &S, 0, sizeof(S));
 	S.q = q; S.m = m; S.n = n;
@@ -1948,19 +2051,7 @@ CPIC_API int cpic_add_species(cpic_ctx_t *c, double q, double m, int64_t n,
 		c->ppt = small || c->precision == CPIC_FP64 ? 1 : kPPT;
 	}
 	int nt = c->ntiles;
-	CK(cudaMalloc(&S.tiles.base, nt * sizeof(int64_t)));
-	CK(cudaMalloc(&S.tiles.cap, nt * sizeof(int32_t)));
-	CK(cudaMalloc(&S.tiles.cnt, nt * sizeof(int32_t)));
-	CK(cudaMalloc(&S.tiles.abase, nt * sizeof(int64_t)));
-	CK(cudaMalloc(&S.tiles.acap, nt * sizeof(int32_t)));
-	CK(cudaMalloc(&S.tiles.acnt[0], nt * sizeof(int32_t)));
-	CK(cudaMalloc(&S.tiles.acnt[1], nt * sizeof(int32_t)));
-	CK(cudaMalloc(&S.tiles.order, nt * sizeof(int32_t)));
-	k_iota<<<grid_blocks(nt), 256, 0, st>>>(nt, S.tiles.order);
-	CK(cudaGetLastError());
-	CK(cudaMemsetAsync(S.tiles.cnt, 0, nt * sizeof(int32_t), st));
-	CK(cudaMemsetAsync(S.tiles.acnt[0], 0, nt * sizeof(int32_t), st));
-	CK(cudaMemsetAsync(S.tiles.acnt[1], 0, nt * sizeof(int32_t), st));
+	if((r = alloc_tiles(S.tiles, nt, st))) return r;
 	// room for an eighth of the species to overflow between two host checks
 	int32_t scap = (int32_t) std::max<int64_t>(65536, n / 8);
 	const int cu = c->precision == CPIC_MIXED ? 1 : 0;

@@ -62,7 +62,7 @@ CPIC_HD int field_node(int t0, int l, int n)
 	return wrapn(t0 + l, n);
 }
 
-// The library's tile size for n particles of one species: the largest of 32,
+// The library's tile size for n particles of one species (the largest): the largest of 32,
 // 16, 8 and 4 cells whose tiles keep the SMs busy to the end.  One block takes
 // a tile, an SM holds 5 or 6 of them, and a block alone on an SM works off
 // its particles at a fraction of the SM's rate, so: over two waves of tiles
