@@ -54,6 +54,7 @@ struct cpic_ctx {
 	cpic_params_t p;
 	Grid g;
 	int ntiles;
+	bool own_tiles;           // the tile size is the library's to choose
 	int ppt;                  // particles per thread of the fused kernel's instance
 	int precision;
 	int64_t iter;
@@ -1767,10 +1768,11 @@ CPIC_API int cpic_create(const cpic_params_t *p, cpic_ctx_t **out)
 	g.idx = 1.0 / g.dx;
 	g.idy = 1.0 / g.dy;
 	// (chosen again as species are added)
-	const int T = p->tile_x > 0 ? p->tile_x
+	c->own_tiles = p->tile_x <= 0 && p->tile_y <= 0;
+	const int T = p->tile_x > 0 ? p->tile_x : p->tile_y > 0 ? p->tile_y
 		: layout::auto_tile(p->nx, p->ny, p->precision == CPIC_FP64, 0);
 	int TY = p->tile_y > 0 ? p->tile_y : T;
-	if(!pow2(T) || !pow2(TY) || (p->tile_x > 0 && (p->nx % T || p->ny % TY)) || T != TY)
+	if(!pow2(T) || !pow2(TY) || (!c->own_tiles && (p->nx % T || p->ny % TY)) || T != TY)
 	{
 		delete c;
 		return CPIC_EINVAL;
@@ -2017,7 +2019,7 @@ CPIC_API int cpic_add_species(cpic_ctx_t *c, double q, double m, int64_t n,
 	// the library's tiles follow the largest species, whatever the order in
 	// which they are added
 	int s = c->nspecies;
-	if(c->p.tile_x <= 0)
+	if(c->own_tiles)
 	{
 		int64_t most = n;
 		for(int k = 0; k < s; k++) most = std::max(most, c->sp[k].n);
