@@ -872,24 +872,12 @@ __global__ void k_f64_to_rho(int64_t n, const double *in, double qscale, long lo
 	}
 }
 
-// The mixed form's fields as FP64: E's two components with the south ghost row
-// (row ny is row 0 again), and phi.
-__global__ void k_E_to_f64(int64_t ng, int64_t ne, const float2 *E, double *ex, double *ey)
-{
-	for(int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; i < ne;
-			i += (int64_t) gridDim.x * blockDim.x)
-	{
-		const float2 v = E[i < ng ? i : i - ng];
-		ex[i] = v.x;
-		ey[i] = v.y;
-	}
-}
-
-__global__ void k_f32_to_f64(int64_t n, const float *in, double *out)
+// Nodes [i0, i0 + n) of every `pitch`-th float from `in` as FP64.
+__global__ void k_f32_to_f64(int64_t i0, int64_t n, const float *in, int pitch, double *out)
 {
 	for(int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n;
 			i += (int64_t) gridDim.x * blockDim.x)
-		out[i] = in[i];
+		out[i] = in[(i0 + i) * pitch];
 }
 
 __global__ void k_iota(int64_t n, int32_t *id)
@@ -1723,6 +1711,7 @@ static int ensure_scratch(cpic_ctx *c, size_t n)
 	if(c->scratch_n >= n) return CPIC_OK;
 	cudaFree(c->scratch);
 	c->scratch = nullptr;
+	c->scratch_n = 0;
 	CK(cudaMalloc(&c->scratch, n * sizeof(double)));
 	c->scratch_n = n;
 	return CPIC_OK;
@@ -2283,6 +2272,25 @@ CPIC_API int cpic_set_rho(cpic_ctx_t *c, const double *rho)
 	return CPIC_OK;
 }
 
+// n nodes of a field of the mixed form into host memory as FP64, widened on the
+// device (on the host, E of a 2048 x 2048 grid took 12 ms) in pieces of the
+// solver's spectrum, which holds nothing between solves: no memory of its own.
+static cudaError_t read_f32(cpic_ctx *c, const float *in, int pitch, int64_t n, double *out)
+{
+	double *d = reinterpret_cast<double *>(c->spec32);
+	const int64_t piece = (int64_t) c->g.ny * (c->g.nx / 2 + 1);
+	for(int64_t i = 0; i < n; i += piece)
+	{
+		const int64_t m = std::min(piece, n - i);
+		k_f32_to_f64<<<grid_blocks(m), 256, 0, c->stream>>>(i, m, in, pitch, d);
+		cudaError_t e = cudaGetLastError();
+		if(e == cudaSuccess)
+			e = cudaMemcpyAsync(out + i, d, m * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
+		if(e != cudaSuccess) return e;
+	}
+	return cudaStreamSynchronize(c->stream);
+}
+
 CPIC_API int cpic_get_phi(cpic_ctx_t *c, double *phi)
 {
 	if(!c || !phi) return CPIC_EINVAL;
@@ -2292,12 +2300,7 @@ CPIC_API int cpic_get_phi(cpic_ctx_t *c, double *phi)
 		CK(cudaMemcpy(phi, c->phi64, ng * sizeof(double), cudaMemcpyDeviceToHost));
 		return CPIC_OK;
 	}
-	// widened on the device: copies at the link's rate, no pass on the host
-	int r = ensure_scratch(c, ng);
-	if(r) return r;
-	k_f32_to_f64<<<grid_blocks(ng), 256, 0, c->stream>>>(ng, c->phi32, c->scratch);
-	CK(cudaMemcpyAsync(phi, c->scratch, ng * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-	CK(cudaStreamSynchronize(c->stream));
+	CK(read_f32(c, c->phi32, 1, ng, phi));
 	return CPIC_OK;
 }
 
@@ -2312,14 +2315,15 @@ CPIC_API int cpic_get_E(cpic_ctx_t *c, double *ex, double *ey)
 		if(ey) CK(cudaMemcpy(ey, c->Ey64, ne * sizeof(double), cudaMemcpyDeviceToHost));
 		return CPIC_OK;
 	}
-	// (on the host, a 2048 x 2048 grid's read-out took 12 ms)
-	int r = ensure_scratch(c, 2 * ne);
-	if(r) return r;
-	double *d = c->scratch;
-	k_E_to_f64<<<grid_blocks(ne), 256, 0, c->stream>>>(ng, ne, c->E32, d, d + ne);
-	if(ex) CK(cudaMemcpyAsync(ex, d, ne * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-	if(ey) CK(cudaMemcpyAsync(ey, d + ne, ne * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-	CK(cudaStreamSynchronize(c->stream));
+	// (row ny is row 0 again)
+	double *out[2] = {ex, ey};
+	for(int k = 0; k < 2; k++)
+	{
+		if(!out[k]) continue;
+		const float *e = &c->E32->x + k;
+		CK(read_f32(c, e, 2, ng, out[k]));
+		memcpy(out[k] + ng, out[k], nx * sizeof(double));
+	}
 	return CPIC_OK;
 }
 
