@@ -2912,10 +2912,11 @@ static int autotune(const cpic_params_t *p, int64_t n, double v0, double vth, bo
 		if(p->nx % T || p->ny % T || (p->nx / T) * (p->ny / T) < 4) continue;
 		for(int P : kPPTChoices)
 		{
-			if(!tune_ppt && P != (fixed > 0 ? fixed : kPPT)) continue;
+			// one pass with the context's own choice (or the caller's)
+			if(!tune_ppt && P != kPPTChoices[0]) continue;
 			cpic_params_t q2 = *p;
 			q2.tile_x = q2.tile_y = T;
-			q2.particles_per_thread = P;
+			q2.particles_per_thread = tune_ppt ? P : fixed;
 			q2.cycles = 0;
 			cpic_ctx_t *c = nullptr;
 			int r = cpic_create(&q2, &c);
