@@ -872,12 +872,14 @@ __global__ void k_f64_to_rho(int64_t n, const double *in, double qscale, long lo
 	}
 }
 
-// Nodes [i0, i0 + n) of every `pitch`-th float from `in` as FP64.
-__global__ void k_f32_to_f64(int64_t i0, int64_t n, const float *in, int pitch, double *out)
+// Component blockIdx.y of `pitch` interleaved FP32 components, n nodes, as FP64,
+// one component after the other.
+__global__ void k_f32_to_f64(int64_t n, const float *in, int pitch, double *out)
 {
+	out += blockIdx.y * n;
 	for(int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n;
 			i += (int64_t) gridDim.x * blockDim.x)
-		out[i] = in[(i0 + i) * pitch];
+		out[i] = in[i * pitch + blockIdx.y];
 }
 
 __global__ void k_iota(int64_t n, int32_t *id)
@@ -2272,23 +2274,39 @@ CPIC_API int cpic_set_rho(cpic_ctx_t *c, const double *rho)
 	return CPIC_OK;
 }
 
-// n nodes of a field of the mixed form into host memory as FP64, widened on the
-// device (on the host, E of a 2048 x 2048 grid took 12 ms) in pieces of the
-// solver's spectrum, which holds nothing between solves: no memory of its own.
-static cudaError_t read_f32(cpic_ctx *c, const float *in, int pitch, int64_t n, double *out)
+// The first nout of a mixed-form field's `pitch` interleaved components, n nodes
+// each, into host memory as FP64, without allocating device memory.  Small ones
+// are widened on the host (E of 16 x 16: 14 us, 27 on the device; 64 x 64: 18 and
+// 27; 128 x 128: 53 and 34; 2048 x 2048: 11 ms and 0.4), the others in the scratch
+// where it holds them, else in the charge buffer that the next particle stage
+// will clear again.
+static cudaError_t read_f32(cpic_ctx *c, const float *in, int pitch, int64_t n, int nout, double *const *out)
 {
-	double *d = reinterpret_cast<double *>(c->spec32);
-	const int64_t piece = (int64_t) c->g.ny * (c->g.nx / 2 + 1);
-	for(int64_t i = 0; i < n; i += piece)
+	cudaStream_t st = c->stream;
+	cudaError_t e = cudaSuccess;
+	if(n <= 4096)
 	{
-		const int64_t m = std::min(piece, n - i);
-		k_f32_to_f64<<<grid_blocks(m), 256, 0, c->stream>>>(i, m, in, pitch, d);
-		cudaError_t e = cudaGetLastError();
-		if(e == cudaSuccess)
-			e = cudaMemcpyAsync(out + i, d, m * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
+		float tmp[2 * 4096];
+		const int64_t m = (n - 1) * pitch + nout;
+		e = cudaMemcpyAsync(tmp, in, m * sizeof(float), cudaMemcpyDeviceToHost, st);
+		if(e == cudaSuccess) e = cudaStreamSynchronize(st);
+		for(int k = 0; k < nout && e == cudaSuccess; k++)
+			for(int64_t i = 0; i < n; i++) out[k][i] = tmp[i * pitch + k];
+		return e;
+	}
+	const bool whole = c->scratch_n >= (size_t) (nout * n);
+	double *d = whole ? c->scratch : reinterpret_cast<double *>(c->rho_buf[c->rho_cur ^ 1]);
+	if(!whole) c->next_clean = false;
+	const int each = whole ? nout : 1;
+	for(int k = 0; k < nout; k += each)
+	{
+		k_f32_to_f64<<<dim3(grid_blocks(n), each), 256, 0, st>>>(n, in + k, pitch, d);
+		e = cudaGetLastError();
+		for(int q = 0; q < each && e == cudaSuccess; q++)
+			e = cudaMemcpyAsync(out[k + q], d + q * n, n * sizeof(double), cudaMemcpyDeviceToHost, st);
 		if(e != cudaSuccess) return e;
 	}
-	return cudaStreamSynchronize(c->stream);
+	return cudaStreamSynchronize(st);
 }
 
 CPIC_API int cpic_get_phi(cpic_ctx_t *c, double *phi)
@@ -2300,7 +2318,7 @@ CPIC_API int cpic_get_phi(cpic_ctx_t *c, double *phi)
 		CK(cudaMemcpy(phi, c->phi64, ng * sizeof(double), cudaMemcpyDeviceToHost));
 		return CPIC_OK;
 	}
-	CK(read_f32(c, c->phi32, 1, ng, phi));
+	CK(read_f32(c, c->phi32, 1, ng, 1, &phi));
 	return CPIC_OK;
 }
 
@@ -2308,22 +2326,19 @@ CPIC_API int cpic_get_E(cpic_ctx_t *c, double *ex, double *ey)
 {
 	if(!c) return CPIC_EINVAL;
 	int64_t nx = c->g.nx, ng = nx * c->g.ny, ne = ng + nx;
-	CK(cudaStreamSynchronize(c->stream));
 	if(c->precision == CPIC_FP64)
 	{
+		CK(cudaStreamSynchronize(c->stream));
 		if(ex) CK(cudaMemcpy(ex, c->Ex64, ne * sizeof(double), cudaMemcpyDeviceToHost));
 		if(ey) CK(cudaMemcpy(ey, c->Ey64, ne * sizeof(double), cudaMemcpyDeviceToHost));
 		return CPIC_OK;
 	}
+	double *const out[2] = {ex ? ex : ey, ey};
+	const int nout = (ex != nullptr) + (ey != nullptr);
+	if(nout > 0) CK(read_f32(c, ex ? &c->E32->x : &c->E32->y, 2, ng, nout, out));
 	// (row ny is row 0 again)
-	double *out[2] = {ex, ey};
-	for(int k = 0; k < 2; k++)
-	{
-		if(!out[k]) continue;
-		const float *e = &c->E32->x + k;
-		CK(read_f32(c, e, 2, ng, out[k]));
+	for(int k = 0; k < nout; k++)
 		memcpy(out[k] + ng, out[k], nx * sizeof(double));
-	}
 	return CPIC_OK;
 }
 

@@ -8,7 +8,7 @@ from cpic_gb300 import _lib
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nx,ny", [(4, 4), (5, 4), (4, 7), (6, 6), (33, 17), (250, 150), (64, 512)])
+@pytest.mark.parametrize("nx,ny", [(4, 4), (5, 4), (4, 7), (6, 6), (33, 17), (250, 150), (64, 64), (241, 17), (64, 512)])
 def test_fields_read_back_exactly(lib, nx, ny):
     rng = np.random.default_rng(nx + 1000 * ny)
     n = 40 * nx * ny
@@ -33,6 +33,29 @@ def test_fields_read_back_exactly(lib, nx, ny):
     ex, ey = c.E()
     assert np.array_equal(ex, wx) and np.array_equal(ey, wy)
     c.close()
+
+
+@pytest.mark.parametrize("nx,ny", [(64, 64), (72, 64), (130, 70)])
+def test_reading_between_the_stages(lib, nx, ny):
+    """Fields read after the field stage leave the particle stage as it is."""
+    rng = np.random.default_rng(3)
+    n = 20 * nx * ny
+    x, y, u, v = rng.random(n) * nx, rng.random(n) * ny, rng.standard_normal(n), rng.standard_normal(n)
+    out = []
+    for read in (False, True):
+        c = _lib.Context(nx, ny, float(nx), float(ny), 0.05, precision=_lib.MIXED)
+        c.add_species(-1.0 / 20, 1.0 / 20, x, y, u, v)
+        c.pre_step()
+        for k in range(3):
+            c.stage_field_E()
+            if read:
+                c.E()
+                c.phi()
+            c.stage_plasma()
+        out.append((c.rho(), *c.E(), *c.particles(0)))
+        c.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
 
 
 def test_reading_takes_no_device_memory(lib):
