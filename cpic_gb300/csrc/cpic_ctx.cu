@@ -47,6 +47,7 @@ struct SpeciesHost {
 	double vmax;              // largest initial |u| component
 	double move;              // mean |dx| + |dy| per step in cells: when loaded,
 	                          // more when a later re-layout finds more
+	layout::Spread spread;    // how evenly it filled the tiles when loaded
 	double wq_mult;           // mixed form: fixed-point units per weight unit
 };
 
@@ -111,6 +112,7 @@ struct cpic_ctx {
 };
 
 constexpr int kCtl = 1 + 2 * kMaxSpecies;
+constexpr int64_t kSpreadSample = 1 << 22;   // particles counted of an upload, at most
 static int32_t *spill_count(const cpic_ctx *c, int list, int s)
 {
 	return c->ctl + 1 + list * kMaxSpecies + s;
@@ -697,8 +699,8 @@ __global__ void k_rb_cursors(int nt, const int64_t *base, const int32_t *neg,
 // Upload check, numbering and Y wrap of a staged species.  out[0]: any
 // invalid record (x outside [0, Lx], non-finite y, ux, uy); out[1]: the
 // largest |ux|, |uy| as the bit pattern of a non-negative double; out[2]: the
-// sum of move_units.
-constexpr int kUploadChk = 3;
+// sum of move_units.  (The other kUploadChk words are k_spread_squares'.)
+constexpr int kUploadChk = 8;
 __global__ void k_upload_check(int64_t n, Spill S, double Lx, double Ly, float cx, float cy,
 		unsigned long long *out)
 {
@@ -732,6 +734,56 @@ __global__ void k_upload_check(int64_t n, Spill S, double Lx, double Ly, float c
 		if(bad) atomicOr(&out[0], 1ULL);
 		if(move) atomicAdd(&out[2], move);
 		atomicMax(&out[1], (unsigned long long) __double_as_longlong(vm));
+	}
+}
+
+// Every step-th particle of a staged species counted into bins of kSpreadBin x
+// kSpreadBin cells (nbx per row; a position outside the box into an edge bin).
+__global__ void k_spread_count(int64_t n, int64_t step, const Spill S, const Grid g, int nbx, int nby,
+		int32_t *bins)
+{
+	const int64_t m = (n + step - 1) / step;
+	for(int64_t i0 = (int64_t) blockIdx.x * blockDim.x; i0 < m; i0 += (int64_t) gridDim.x * blockDim.x)
+	{
+		const int64_t i = i0 + threadIdx.x;
+		const bool on = i < m;
+		int b = 0;
+		if(on)
+		{
+			const int cx = (int) (S.x[i * step] * g.idx), cy = (int) (S.y[i * step] * g.idy);
+			b = min(max(cy / layout::kSpreadBin, 0), nby - 1) * nbx
+				+ min(max(cx / layout::kSpreadBin, 0), nbx - 1);
+		}
+		warp_reserve(bins, on, b);
+	}
+}
+
+// out[k]: sum over the tiles of 1 << k bins a side of their counts' squares
+// (blockIdx.y = k); out[4]: the particles counted.
+__global__ void k_spread_squares(int nbx, int nby, const int32_t *bins, unsigned long long *out)
+{
+	const int k = blockIdx.y, w = 1 << k;
+	const int ntx = (nbx + w - 1) >> k, nty = (nby + w - 1) >> k;
+	unsigned long long sum = 0, num = 0;
+	for(int64_t t = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; t < (int64_t) ntx * nty;
+			t += (int64_t) gridDim.x * blockDim.x)
+	{
+		const int ty = (int) (t / ntx), tx = (int) (t - (int64_t) ty * ntx);
+		unsigned long long c = 0;
+		for(int y = ty << k; y < min((ty + 1) << k, nby); y++)
+			for(int x = tx << k; x < min((tx + 1) << k, nbx); x++) c += bins[(int64_t) y * nbx + x];
+		sum += c * c;
+		num += c;
+	}
+	for(int o = 16; o > 0; o >>= 1)
+	{
+		sum += __shfl_xor_sync(0xffffffffu, sum, o);
+		num += __shfl_xor_sync(0xffffffffu, num, o);
+	}
+	if((threadIdx.x & 31) == 0 && num)
+	{
+		atomicAdd(&out[k], sum);
+		if(k == 0) atomicAdd(&out[4], num);
 	}
 }
 
@@ -1985,7 +2037,7 @@ CPIC_API int cpic_add_species(cpic_ctx_t *c, double q, double m, int64_t n,
 	Spill stg;
 	memset(&stg, 0, sizeof(stg));
 	if((r = alloc_spill(stg, (int32_t) std::max<int64_t>(n, 1), st))) return r;
-	double vmax = 0.0, move = 0.0;
+	double vmax = 0.0, move = 0.0, counted = 0.0, squares[4] = {0.0, 0.0, 0.0, 0.0};
 	if(n > 0)
 	{
 		CK(cudaMemcpyAsync(stg.x, x, n * sizeof(double), cudaMemcpyHostToDevice, st));
@@ -1996,6 +2048,20 @@ CPIC_API int cpic_add_species(cpic_ctx_t *c, double q, double m, int64_t n,
 		CK(cudaMemsetAsync(c->upload_chk, 0, sizeof(h), st));
 		k_upload_check<<<grid_blocks(n, 256, 8 * 152), 256, 0, st>>>(n, stg, c->p.Lx, c->p.Ly,
 				move_cx(c), move_cy(c), c->upload_chk);
+		if(c->own_tiles)
+		{
+			// counted in the charge buffer that the next particle stage clears
+			const int nbx = (c->g.nx + layout::kSpreadBin - 1) / layout::kSpreadBin;
+			const int nby = (c->g.ny + layout::kSpreadBin - 1) / layout::kSpreadBin;
+			int32_t *bins = reinterpret_cast<int32_t *>(c->rho_buf[c->rho_cur ^ 1]);
+			const int64_t step = (n + kSpreadSample - 1) / kSpreadSample;
+			c->next_clean = false;
+			CK(cudaMemsetAsync(bins, 0, (size_t) nbx * nby * sizeof(int32_t), st));
+			k_spread_count<<<grid_blocks((n + step - 1) / step), 256, 0, st>>>(n, step, stg, c->g, nbx, nby, bins);
+			k_spread_squares<<<dim3(grid_blocks((int64_t) nbx * nby, 256, 1024), 4), 256, 0, st>>>(nbx, nby, bins,
+					c->upload_chk + 3);
+			CK(cudaGetLastError());
+		}
 		CK(cudaMemcpyAsync(h, c->upload_chk, sizeof(h), cudaMemcpyDeviceToHost, st));
 		CK(cudaStreamSynchronize(st));
 		if(h[0])
@@ -2005,16 +2071,27 @@ CPIC_API int cpic_add_species(cpic_ctx_t *c, double q, double m, int64_t n,
 		}
 		memcpy(&vmax, &h[1], sizeof(double));
 		move = (double) h[2] / kMoveUnits / (double) n;
+		for(int k = 0; k < 4; k++) squares[k] = (double) h[3 + k];
+		counted = (double) h[7];
 	}
 
 	// the library's tiles follow the largest species, whatever the order in
-	// which they are added
+	// which they are added: the smallest of the tiles that suit those of at
+	// least half its particles
 	int s = c->nspecies;
+	const layout::Spread spread = layout::spread(c->p.nx, c->p.ny, counted, squares);
 	if(c->own_tiles)
 	{
+		const bool f64 = c->precision == CPIC_FP64;
 		int64_t most = n;
 		for(int k = 0; k < s; k++) most = std::max(most, c->sp[k].n);
-		const int T = layout::auto_tile(c->p.nx, c->p.ny, c->precision == CPIC_FP64, most);
+		int T = 32;
+		for(int k = 0; k <= s; k++)
+		{
+			const int64_t nk = k < s ? c->sp[k].n : n;
+			if(nk >= most - nk)
+				T = std::min(T, layout::uneven_tile(c->p.nx, c->p.ny, f64, nk, k < s ? c->sp[k].spread : spread));
+		}
 		if(T != c->g.tx && (r = change_tiles(c, T)))
 		{
 			free_spill(stg);
@@ -2026,6 +2103,7 @@ CPIC_API int cpic_add_species(cpic_ctx_t *c, double q, double m, int64_t n,
 	S.q = q; S.m = m; S.n = n;
 	S.vmax = vmax;
 	S.move = move;
+	S.spread = spread;
 	// the fused kernel's instance when the caller left it to the library.
 	// FP64: 1 particle per thread; the kernel's arithmetic is long enough to
 	// hide a chunk's latency, and a second copy of its code misses the

@@ -62,7 +62,12 @@ CPIC_HD int field_node(int t0, int l, int n)
 	return wrapn(t0 + l, n);
 }
 
-// The library's tile size for n particles of one species (the largest): the largest of 32,
+inline int64_t tiles_of(int64_t nx, int64_t ny, int T)
+{
+	return ((nx + T - 1) / T) * ((ny + T - 1) / T);
+}
+
+// The library's tile size for n evenly spread particles of one species: the largest of 32,
 // 16, 8 and 4 cells whose tiles keep the SMs busy to the end.  One block takes
 // a tile, an SM holds 5 or 6 of them, and a block alone on an SM works off
 // its particles at a fraction of the SM's rate, so: over two waves of tiles
@@ -86,13 +91,73 @@ inline int auto_tile(int64_t nx, int64_t ny, bool f64, int64_t n)
 	while(T >= 2 * nx || T >= 2 * ny) T >>= 1;
 	for(; T > 4; T >>= 1)
 	{
-		const int64_t tiles = ((nx + T - 1) / T) * ((ny + T - 1) / T);
+		const int64_t tiles = tiles_of(nx, ny, T);
 		const int64_t per = n / tiles;
 		if(tiles >= 2048 || (tiles >= 912 && per <= (f64 ? 2048 : 8192))
 				|| (tiles >= 152 && per <= (f64 ? 512 : 1024)) || per <= 128)
 			return T;
 	}
 	return 4;
+}
+
+// How evenly a species fills the tiles: for tiles of 4, 8, 16 and 32 cells
+// (index log2 T - 2) the number of equal tiles with the same load as a particle
+// sees on average, (sum c)^2 / (sum c^2 - sum c) for tiles of c particles (the
+// subtraction takes out chance: evenly scattered particles give the number of
+// tiles).
+struct Spread { double tiles[4]; };
+constexpr int kSpreadBin = 4;                  // cells per side of a counted bin
+
+inline Spread spread(int64_t nx, int64_t ny, double count, const double squares[4])
+{
+	Spread e;
+	for(int k = 0; k < 4; k++)
+	{
+		e.tiles[k] = (double) tiles_of(nx, ny, kSpreadBin << k);
+		if(squares[k] > count)
+			e.tiles[k] = std::min(e.tiles[k], count * count / (squares[k] - count));
+	}
+	return e;
+}
+
+// Time of the particle kernel on n unevenly spread particles, us: a share for
+// every tile, most of them empty, over the blocks that the GPU holds, and the
+// heavy tiles' particles, which one block works off.  Fitted to a sweep of 140
+// loads (boxes, a bell, half of the particles in a tenth of the grid, a sine;
+// 64^2 to 2048^2 cells, 0.26 to 8 million particles, 4 tile sizes each).
+inline double uneven_cost(int64_t nx, int64_t ny, bool f64, int64_t n, int T, double tiles)
+{
+	const double all = (double) tiles_of(nx, ny, T) / 912 * (1.0 + T * T / 800.0);
+	const double load = (double) n / std::max(tiles, 1.0);
+	return f64 ? 10.0 + 4.6 * all + 61e-6 * n + 32e-3 * load : 9.0 + 3.1 * all + 6.8e-6 * n + 5.8e-3 * load;
+}
+
+// The tile size for n particles spread as e says: that of an even load, unless
+// fewer than three quarters of those tiles carry it and a smaller tile costs at
+// most 0.85 as much by uneven_cost.  Particle kernel, us, with the even load's
+// tile, with the tile chosen here and with the best of the four: mixed 512 x 512,
+// 4 million in a fifth of each side 299, 83, 83; a bell of a tenth of the side
+// 189, 83, 83; 1024 x 1024, 2 million in a fifth 145, 56, 56; 2048 x 2048, 8
+// million, a bell 122 (kept), 122; FP64 256 x 256, 2 million in a fifth 1148,
+// 348, 348; 1024 x 1024, 8 million, half in a tenth 585 (kept), 585.  Over the
+// sweep the worst choice is 1.15 times the best (27 us instead of 24).
+inline int uneven_tile(int64_t nx, int64_t ny, bool f64, int64_t n, const Spread &e)
+{
+	int T = auto_tile(nx, ny, f64, n), k = 0;
+	while(kSpreadBin << k < T) k++;
+	if(e.tiles[k] >= 0.75 * (double) tiles_of(nx, ny, T))
+		return T;
+	double least = 0.85 * uneven_cost(nx, ny, f64, n, T, e.tiles[k]);
+	while(--k >= 0)
+	{
+		const double cost = uneven_cost(nx, ny, f64, n, kSpreadBin << k, e.tiles[k]);
+		if(cost < least)
+		{
+			least = cost;
+			T = kSpreadBin << k;
+		}
+	}
+	return T;
 }
 
 // Room for arrivals in percent of a tile's particles, for a species that moves

@@ -65,7 +65,8 @@ typedef struct cpic_params {
 	int32_t tile_x, tile_y;  /* cells per tile, equal powers of two dividing
 	                          * nx and ny (one given holds for both); 0 = chosen
 	                          * by the number of particles of the largest
-	                          * species, need not divide the grid */
+	                          * species and how evenly they are spread, need
+	                          * not divide the grid */
 	int32_t halo;            /* deposit halo in cells; 0 = auto */
 	int32_t track_ids;       /* keep a particle id per particle (MIXED) */
 	int32_t particles_per_thread; /* fused kernel instance: 1, 2 or 4; 0 = chosen
