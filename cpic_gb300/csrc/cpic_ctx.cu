@@ -1883,7 +1883,12 @@ CPIC_API int cpic_create(const cpic_params_t *p, cpic_ctx_t **out)
 	int64_t nh = g.nx / 2 + 1;
 	int r = CPIC_OK;
 #define AL(ptr, bytes) do { if(cudaMalloc(&(ptr), (bytes)) != cudaSuccess) { r = CPIC_ENOMEM; goto fail; } } while(0)
-	for(int k = 0; k < 2; k++) AL(c->rho_buf[k], ng * sizeof(long long));
+	// the charge buffers together (an allocation takes tens of us)
+	const int64_t nrho = (ng + 31) & ~(int64_t) 31;
+	AL(c->rho_buf[0], (p->precision == CPIC_FP64 ? 4 : 2) * nrho * sizeof(long long));
+	c->rho_buf[1] = c->rho_buf[0] + nrho;
+	for(int k = 0; k < 2 && p->precision == CPIC_FP64; k++)
+		c->rho_lo_buf[k] = c->rho_buf[0] + (2 + k) * nrho;
 	AL(c->ctl, kCtl * sizeof(int32_t));
 	c->status = reinterpret_cast<uint32_t *>(c->ctl);
 	AL(c->cosx, g.nx * sizeof(double));
@@ -1894,7 +1899,6 @@ CPIC_API int cpic_create(const cpic_params_t *p, cpic_ctx_t **out)
 	if(c->precision == CPIC_FP64)
 	{
 		AL(c->phi64, ng * sizeof(double));
-		for(int k = 0; k < 2; k++) AL(c->rho_lo_buf[k], ng * sizeof(long long));
 		AL(c->Ex64, (ng + 3 * (int64_t) g.nx) * sizeof(double));
 		AL(c->Ey64, (ng + 3 * (int64_t) g.nx) * sizeof(double));
 		AL(c->spec64, ng / g.nx * nh * sizeof(double2));
@@ -1990,7 +1994,7 @@ CPIC_API void cpic_destroy(cpic_ctx_t *c)
 		free_spill(S.spill[0], false);
 		free_spill(S.spill[1], false);
 	}
-	for(int k = 0; k < 2; k++) { cudaFree(c->rho_buf[k]); cudaFree(c->rho_lo_buf[k]); }
+	cudaFree(c->rho_buf[0]);
 	cudaFree(c->phi64); cudaFree(c->Ex64); cudaFree(c->Ey64);
 	cudaFree(c->phi32); cudaFree(c->E32); cudaFree(c->spec64); cudaFree(c->spec32);
 	cudaFree(c->twx64); cudaFree(c->twy64); cudaFree(c->twx32); cudaFree(c->twy32);
