@@ -1362,9 +1362,16 @@ CPIC_API int cpic_adj_create(const cpic_adj_params_t *p, int64_t n, cpic_adj_t *
 	a->idx_ok = bits::pos_of(a->g.idx, a->g.idx_p) & bits::pos_of(a->g.idy, a->g.idy_p);
 	// Particles per block: enough blocks for the SMs to finish together (four
 	// or five are resident on each), else as many as amortise the region's
-	// flush.  FP64 (whose particles take longest), 1,048,576 of them on 128 x
-	// 128, 200 steps: 2048 per block 73.0 ms, 1024 63.8, 512 60.6; FP32,
-	// 262,144 on 64 x 64, 50 steps: 1024 5.16 ms, 512 4.84, 256 4.99.
+	// flush.  Forward and reverse of 20 steps, ms, with 256, 512, 1024 and 2048
+	// per block: FP64 (whose particles take longest) 140,000 on 128 x 128
+	// 2.95, 3.22, 3.52, 3.95; 300,000 3.50, 3.74, 4.54, 4.91; 1,048,576 6.52,
+	// 6.44, 6.58, 7.52; 3,145,728 on 256 x 256 16.3, 15.6, 15.5, 16.3; 5,242,880
+	// 26.0, 24.7, 24.1, 24.6; 10,485,760 on 512 x 512 53.4, 50.6, 49.2, 49.5.
+	// FP32 70,000 on 64 x 64 1.38, 1.44, 1.54, 1.91; 150,000 1.56, 1.56, 1.68,
+	// 1.90; 600,000 on 128 x 128 2.64, 2.48, 2.70, 3.19; 1,572,864 4.57, 4.07,
+	// 3.95, 4.13; 3,145,728 on 256 x 256 8.38, 7.25, 6.83, 6.89; 5,242,880 13.5,
+	// 11.6, 10.7, 10.4.  (The FP64 limits at 150,000 and 8 million lie a few per
+	// cent from where the curves cross.)
 	if(a->f64)
 		a->chunk = n >= 8 << 20 ? 2048 : n >= 4 << 20 ? 1024 : n >= 150000 ? 512 : 256;
 	else

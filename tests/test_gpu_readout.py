@@ -60,6 +60,10 @@ def test_reading_between_the_stages(lib, nx, ny):
 
 def test_reading_takes_no_device_memory(lib):
     torch = pytest.importorskip("torch")
+    warm = _lib.Context(128, 128, 1.0, 1.0, 1e-3, precision=_lib.MIXED)     # (loads the kernels)
+    warm.E()
+    warm.phi()
+    warm.close()
     c = _lib.Context(1024, 1024, 1.0, 1.0, 1e-3, precision=_lib.MIXED)
     c.add_species(-1.0, 1.0, [0.5], [0.5], [0.0], [0.0])
     c.pre_step()
