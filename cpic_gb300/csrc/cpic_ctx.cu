@@ -1271,8 +1271,8 @@ static float move_cy(const cpic_ctx *c) { return (float) (c->p.dt * c->g.idy); }
 // 4 ints per tile in shared memory: 128 KB).
 constexpr int kBlkSortMaxTiles = 8192;
 
-// Counting-sort rebuild of species s: its tiles (unless `fresh`), its
-// current spill input and an optional staging list are merged into a new
+// Counting-sort rebuild of species s: its tiles and its current spill input
+// (unless `fresh`) and an optional staging list are merged into a new
 // layout whose tile capacities follow the new counts and the species' speed,
 // which is measured again if `measure` says so.
 static int rebuild_species(cpic_ctx *c, int s, bool fresh, const Spill *staging, int64_t nstage,
@@ -1282,10 +1282,15 @@ static int rebuild_species(cpic_ctx *c, int s, bool fresh, const Spill *staging,
 	int nt = c->ntiles;
 	cudaStream_t st = c->stream;
 	Spill &spin = S.spill[c->spill_cur];
+	// (a fresh layout holds the staged particles only: what the spill list
+	// held of the old ones goes with them)
 	int32_t nspill = 0;
-	CK(cudaMemcpyAsync(&nspill, spin.count, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-	CK(cudaStreamSynchronize(st));
-	if(nspill > spin.capacity) nspill = spin.capacity;
+	if(!fresh)
+	{
+		CK(cudaMemcpyAsync(&nspill, spin.count, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+		CK(cudaStreamSynchronize(st));
+		if(nspill > spin.capacity) nspill = spin.capacity;
+	}
 
 	// the new counts, then two 64-bit words: how far the particles move (measure)
 	const int ntp = (nt + 1) & ~1;
@@ -1311,7 +1316,7 @@ static int rebuild_species(cpic_ctx *c, int s, bool fresh, const Spill *staging,
 	bool mix = c->precision == CPIC_MIXED;
 	// the upload of a species: one conversion pass (records, keys and the
 	// histogram of (tile, sign of ux)), then two sorting passes below
-	const bool blk = fresh && staging && nspill == 0 && nstage > 0 && nt <= kBlkSortMaxTiles;
+	const bool blk = fresh && staging && nstage > 0 && nt <= kBlkSortMaxTiles;
 	const int blk_blocks = (int) std::min<int64_t>(152 * 8, (nstage + 4095) / 4096);
 	SpeciesHost tmp1, tmp2;
 	memset((void *) &tmp1, 0, sizeof(tmp1));
