@@ -957,14 +957,15 @@ __global__ void k_f64_to_rho(int64_t n, const double *in, double qscale, long lo
 	}
 }
 
-// Component blockIdx.y of `pitch` interleaved FP32 components, n nodes, as FP64,
-// one component after the other.
-__global__ void k_f32_to_f64(int64_t n, const float *in, int pitch, double *out)
+// Component blockIdx.y of `pitch` interleaved FP32 components as FP64, one
+// component after the other: n nodes, those past the ng of the grid the first
+// ones again.
+__global__ void k_f32_to_f64(int64_t ng, int64_t n, const float *in, int pitch, double *out)
 {
 	out += blockIdx.y * n;
 	for(int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x; i < n;
 			i += (int64_t) gridDim.x * blockDim.x)
-		out[i] = in[i * pitch + blockIdx.y];
+		out[i] = in[(i < ng ? i : i - ng) * pitch + blockIdx.y];
 }
 
 __global__ void k_iota(int64_t n, int32_t *id)
@@ -1888,8 +1889,9 @@ CPIC_API int cpic_create(const cpic_params_t *p, cpic_ctx_t **out)
 	int64_t nh = g.nx / 2 + 1;
 	int r = CPIC_OK;
 #define AL(ptr, bytes) do { if(cudaMalloc(&(ptr), (bytes)) != cudaSuccess) { r = CPIC_ENOMEM; goto fail; } } while(0)
-	// the charge buffers together (an allocation takes tens of us)
-	const int64_t nrho = (ng + 31) & ~(int64_t) 31;
+	// the charge buffers together (an allocation takes tens of us), each with a
+	// row to spare (read_f32)
+	const int64_t nrho = (ng + g.nx + 31) & ~(int64_t) 31;
 	AL(c->rho_buf[0], (p->precision == CPIC_FP64 ? 4 : 2) * nrho * sizeof(long long));
 	c->rho_buf[1] = c->rho_buf[0] + nrho;
 	for(int k = 0; k < 2 && p->precision == CPIC_FP64; k++)
@@ -2397,24 +2399,27 @@ CPIC_API int cpic_set_rho(cpic_ctx_t *c, const double *rho)
 	return CPIC_OK;
 }
 
-// The first nout of a mixed-form field's `pitch` interleaved components, n nodes
-// each, into host memory as FP64, without allocating device memory.  Small ones
+// The first nout of a mixed-form field's `pitch` interleaved components into host
+// memory as FP64, n nodes each (the ng of the grid, then the first row again),
+// without allocating device memory.  Small ones
 // are widened on the host (E of 16 x 16: 14 us, 27 on the device; 64 x 64: 18 and
 // 27; 128 x 128: 53 and 34; 2048 x 2048: 11 ms and 0.4), the others in the scratch
 // where it holds them, else in the charge buffer that the next particle stage
-// will clear again.
+// will clear again.  (The repeated row comes in the same copy: written by the
+// host, it took 1.5 ms more of a 2048 x 2048 read-out into fresh memory.)
 static cudaError_t read_f32(cpic_ctx *c, const float *in, int pitch, int64_t n, int nout, double *const *out)
 {
+	const int64_t ng = (int64_t) c->g.nx * c->g.ny;
 	cudaStream_t st = c->stream;
 	cudaError_t e = cudaSuccess;
-	if(n <= 4096)
+	if(ng <= 4096)
 	{
 		float tmp[2 * 4096];
-		const int64_t m = (n - 1) * pitch + nout;
+		const int64_t m = (ng - 1) * pitch + nout;
 		e = cudaMemcpyAsync(tmp, in, m * sizeof(float), cudaMemcpyDeviceToHost, st);
 		if(e == cudaSuccess) e = cudaStreamSynchronize(st);
 		for(int k = 0; k < nout && e == cudaSuccess; k++)
-			for(int64_t i = 0; i < n; i++) out[k][i] = tmp[i * pitch + k];
+			for(int64_t i = 0; i < n; i++) out[k][i] = tmp[(i < ng ? i : i - ng) * pitch + k];
 		return e;
 	}
 	const bool whole = c->scratch_n >= (size_t) (nout * n);
@@ -2423,7 +2428,7 @@ static cudaError_t read_f32(cpic_ctx *c, const float *in, int pitch, int64_t n, 
 	const int each = whole ? nout : 1;
 	for(int k = 0; k < nout; k += each)
 	{
-		k_f32_to_f64<<<dim3(grid_blocks(n), each), 256, 0, st>>>(n, in + k, pitch, d);
+		k_f32_to_f64<<<dim3(grid_blocks(n), each), 256, 0, st>>>(ng, n, in + k, pitch, d);
 		e = cudaGetLastError();
 		for(int q = 0; q < each && e == cudaSuccess; q++)
 			e = cudaMemcpyAsync(out[k + q], d + q * n, n * sizeof(double), cudaMemcpyDeviceToHost, st);
@@ -2458,10 +2463,8 @@ CPIC_API int cpic_get_E(cpic_ctx_t *c, double *ex, double *ey)
 	}
 	double *const out[2] = {ex ? ex : ey, ey};
 	const int nout = (ex != nullptr) + (ey != nullptr);
-	if(nout > 0) CK(read_f32(c, ex ? &c->E32->x : &c->E32->y, 2, ng, nout, out));
 	// (row ny is row 0 again)
-	for(int k = 0; k < nout; k++)
-		memcpy(out[k] + ng, out[k], nx * sizeof(double));
+	if(nout > 0) CK(read_f32(c, ex ? &c->E32->x : &c->E32->y, 2, ne, nout, out));
 	return CPIC_OK;
 }
 
